@@ -357,17 +357,29 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
     }
     const int npi = (int)cls.size();
     std::vector<int> cl_start(npi + 1), cl_index, blk_start(nat * nat + 1, 0);
+    std::vector<int> cls_grp(npi + 1), grp_start, grp_a2;  // 4ph: runs of one second atom within each class
     std::vector<int4> pi_d(npi);
     int p = 0;
     for (auto& kv : cls) {
         cl_start[p] = (int)cl_index.size();
-        for (int t : kv.second) cl_index.push_back(t);
+        if (order == 4)
+            std::stable_sort(kv.second.begin(), kv.second.end(), [&](int x, int y) { return atoms[x].y < atoms[y].y; });
+        cls_grp[p] = (int)grp_start.size();
+        for (int t : kv.second) {
+            if ((int)grp_start.size() == cls_grp[p] || grp_a2.back() != atoms[t].y) {
+                grp_start.push_back((int)cl_index.size());
+                grp_a2.push_back(atoms[t].y);
+            }
+            cl_index.push_back(t);
+        }
         pi_d[p] = make_int4(std::get<1>(kv.first), std::get<2>(kv.first), std::get<3>(kv.first),
                             std::get<4>(kv.first) * 256 + std::get<5>(kv.first));
         blk_start[std::get<0>(kv.first) + 1]++;
         p++;
     }
     cl_start[npi] = (int)cl_index.size();
+    cls_grp[npi] = (int)grp_start.size();
+    grp_start.push_back((int)cl_index.size());
     for (int b = 0; b < nat * nat; b++) blk_start[b + 1] += blk_start[b];
     int r;
     if ((r = T.phi.upload(c, ph.data(), ph.size() * sizeof(double)))) return r;
@@ -380,6 +392,11 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
     if ((r = T.cl_index.upload(c, cl_index.data(), ntri * sizeof(int)))) return r;
     if ((r = T.pi_d.upload(c, pi_d.data(), npi * sizeof(int4)))) return r;
     if ((r = T.blk_start.upload(c, blk_start.data(), (nat * nat + 1) * sizeof(int)))) return r;
+    if (order == 4) {
+        if ((r = T.cls_grp.upload(c, cls_grp.data(), cls_grp.size() * sizeof(int)))) return r;
+        if ((r = T.grp_start.upload(c, grp_start.data(), grp_start.size() * sizeof(int)))) return r;
+        if ((r = T.grp_a2.upload(c, grp_a2.data(), grp_a2.size() * sizeof(int)))) return r;
+    }
     T.h_blk_start = blk_start;
     DevIfc& F = T.F;
     F.order = order;
@@ -394,6 +411,9 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
     F.mu = T.mu.as<double>();
     F.cl_start = T.cl_start.as<int>();
     F.cl_index = T.cl_index.as<int>();
+    F.cls_grp = T.cls_grp.as<int>();
+    F.grp_start = T.grp_start.as<int>();
+    F.grp_a2 = T.grp_a2.as<int>();
     F.pi_d = T.pi_d.as<int4>();
     F.blk_start = T.blk_start.as<int>();
     return FP4_OK;

@@ -45,6 +45,9 @@ struct DevIfc {
     const double* mu;            // 1/sqrt(product of masses)
     const int* cl_start;         // clusters sorted by class: class p owns [cl_start[p], cl_start[p+1])
     const int* cl_index;         // cluster ids in class order
+    const int* cls_grp;          // 4ph: class p's clusters in groups of one second atom, groups [cls_grp[p], cls_grp[p+1])
+    const int* grp_start;        // 4ph: group g owns cl_index[grp_start[g] .. grp_start[g+1])
+    const int* grp_a2;           // 4ph: second atom of group g
     const int4* pi_d;            // class displacement D (x,y,z) and packed atom pair in .w
     const int* blk_start;        // classes sorted by atom-pair block: block b owns [blk_start[b], blk_start[b+1])
 };

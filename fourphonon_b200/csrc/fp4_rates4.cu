@@ -8,7 +8,8 @@
 //     exact operation order (computed once for all (i,j)), a binary search for
 //     the window of s_ij that can pass the 1-sigma test, and the exact test in
 //     the reference's operation order.  Survivors are queued per (i,j);
-//   * phase B builds, per branch i, the reciprocal cluster table
+//   * phase B (a function of its own, with its own registers) builds, per branch i, the
+//     reciprocal cluster table
 //         Z_p^{(ij)}[s][r] = sum_{c in p} kappa_c sum_{u,t} Psi_c[u][t][s][r] e_i[u] e~'_j[t]
 //     and contracts each queued process as
 //         V = sum_p w_p(q'') e~''_k[s] Z_p[s][r] conj(e'''_l[r]),
@@ -19,6 +20,13 @@
 //     temperature of the call; |V|^2 is formed once for all of them.
 // Per-(work item, branch, temperature) partial sums are reduced afterwards in
 // a fixed order with compensated summation (k4_reduce).
+//
+// What bounds it (12^3 diamond, FP64, two temperatures; 1.09 s before phase B's tables,
+// loads and sums were rearranged, 1.02 s after): no single unit.  Builds that leave one
+// part out put the class loop at 40 % of phase B, the gathers of the two eigenvector
+// rows at 16 %, the weights at 16 %, the tables at 5 %; a warp's chain of dependent
+// loads and FP64 operations is exposed at 16 warps per SM, and a third CTA per SM (80
+// registers, spills, a smaller L1) is slower (1.19 s).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -43,7 +51,6 @@ constexpr int kCheckEvery = 8;  // list mode: passes between queue-capacity chec
 // The multi-solve kernel keeps more state per thread (the slot, its layout) and runs
 // two CTAs per SM in both precisions: at three the FP32 form spills.
 constexpr int kMultiCtasPerSm = 2;
-
 template <int KIND, int NT, bool MIXED>
 constexpr int ctas_per_sm() {
     return (KIND == 0 || (MIXED && NT <= 2)) ? 3 : 2;
@@ -73,11 +80,20 @@ struct CT<true> {
 };
 
 struct Layout {
-    size_t z, kap, pt, sval, swj, racc, wacc, pacc, red, sidx, cnt, ncnt, klt, pre, blk, seg, jjl, stg, stgi, misc,
-        total;
+    int z, kap, pt, cfl, sval, swj, racc, wacc, pacc, red, sidx, cnt, ncnt, klt, pre, blk, seg, jjl, stg, stgi,
+        misc, total;
     int allz;  // 1: the reciprocal cluster tables of all (i,j) at once, 0: one branch i at a time
+    int bgrp;  // capacity (cluster groups) of the staging area when phase B builds its tables there
     int njjl;  // capacity of the list of q'' that the channel's restriction keeps (0: no list)
     int stgp;  // phase-A passes per stage of (v, omega) records
+};
+
+// What phase B reads of the kernel's arguments, at the start of dynamic shared memory:
+// phase B is a function of its own, so that its registers are not shared with the
+// state that phase A keeps across a drain of the queues.
+struct K4Shared {
+    P4Params p;
+    Layout L;
 };
 
 // Phase A stages the (v, omega) records of the third phonon's grid points of the
@@ -111,52 +127,57 @@ __host__ __device__ inline Layout k4_layout_z(int kind, int NT, bool mixed, int 
     L.njjl = njjl;
     const size_t cs = mixed ? 8 : 16;  // complex size
     const size_t nb2 = (size_t)nb * nb;
-    size_t o = 0;
-    L.z = o;
+    size_t o = noz ? 0 : al16(sizeof(K4Shared));
+    L.z = (int)o;
     o = al16(o + ((kind >= 2 && !noz) ? (allz ? nb2 : (size_t)nb) * npi * 9 * cs : 0));
-    L.kap = o;
+    L.kap = (int)o;
     o = al16(o + ((kind >= 2) ? (size_t)ntri * 16 : 0));
-    L.pt = o;
+    L.pt = (int)o;
     o = al16(o + ((kind >= 2) ? (size_t)npi * lsum * cs : 0));
-    L.sval = o;
+    L.cfl = (int)o;  // per class: the axes (bits 0-2) along which its phase is not 1
+    o = al16(o + ((kind >= 2 && !noz) ? (size_t)npi : 0));
+    L.sval = (int)o;
     o = al16(o + nb2 * 8);
-    L.swj = o;  // omega'_j of each sorted pair
+    L.swj = (int)o;  // omega'_j of each sorted pair
     o = al16(o + nb2 * 8);
-    L.racc = o;
+    L.racc = (int)o;
     o = al16(o + (size_t)nb * NT * 8);
-    L.wacc = o;
+    L.wacc = (int)o;
     o = al16(o + (size_t)nb * NT * 8);
     // counting: one copy of the per-branch count and phase-space sum per warp, so that
     // the shared-memory atomics of a survivor contend within its warp only
     const size_t ncopy = (kind == 0) ? kThreads / 32 : 1;
-    L.pacc = o;
+    L.pacc = (int)o;
     o = al16(o + (size_t)nb * ncopy * 8);
-    L.red = o;  // block_sum_vec of 2*NT values (phase B) or 4 (work counters)
-    o = al16(o + (size_t)32 * (2 * NT > 4 ? 2 * NT : 4) * 8);
-    L.sidx = o;
+    L.red = (int)o;  // block_sum_vec of the 4 work counters
+    o = al16(o + (size_t)32 * 4 * 8);
+    L.sidx = (int)o;
     o = al16(o + nb2 * 4);
-    L.cnt = o;
+    L.cnt = (int)o;
     o = al16(o + nb2 * 4);
-    L.ncnt = o;
+    L.ncnt = (int)o;
     o = al16(o + (size_t)nb * ncopy * 4);
-    L.klt = o;
+    L.klt = (int)o;
     o = al16(o + nb2 * 4);
-    L.pre = o;
-    o = al16(o + (nb2 + 1) * 4);
-    L.blk = o;  // non-empty atom-pair blocks of the class table: (first class, end, atom k, atom l)
-    o = al16(o + (size_t)(kMaxNb / 3) * (kMaxNb / 3) * 16);
-    L.seg = o;  // kind 3: first list position of each branch's q' segment, then the segments' prefix
-    o = al16(o + (size_t)(2 * nb + 1) * 8);
-    L.jjl = o;
+    // phase B's prefix of the entries over the bins of one group
+    const size_t gbins = noz ? 0 : (allz ? nb2 : (size_t)nb);
+    L.pre = (int)o;
+    o = al16(o + (kind >= 2 ? (gbins + 1) * 4 : 0));
+    L.blk = (int)o;  // non-empty atom-pair blocks of the class table: (first class, end, atom k, atom l)
+    o = al16(o + (kind >= 2 ? (size_t)(nb / 3) * (nb / 3) * 16 : 0));
+    L.seg = (int)o;  // kind 3: first list position of each branch's q' segment, then the segments' prefix
+    o = al16(o + (kind == 3 ? (size_t)(2 * nb + 1) * 8 : 0));
+    L.jjl = (int)o;
     o = al16(o + (size_t)njjl * 2 + 32 * 4);  // the list, then per-warp counts of the compaction
     L.stgp = stage_passes((int)nb2);
-    L.stg = o;  // per staged point: the records (v, omega) of its nb branches, then those of its partner
+    L.stg = (int)o;  // per staged point: the records (v, omega) of its nb branches, then those of its partner
     o = al16(o + (size_t)stage_slots((int)nb2) * 2 * nb * 32);
-    L.stgi = o;  // per staged point: (its index, its grid coordinates packed, the partner's index)
+    L.bgrp = stage_slots((int)nb2) * 2 * nb * 32 / (27 * 16);  // cluster groups that fit there in phase B
+    L.stgi = (int)o;  // per staged point: (its index, its grid coordinates packed, the partner's index)
     o = al16(o + (size_t)stage_slots((int)nb2) * 16);
-    L.misc = o;
+    L.misc = (int)o;
     o = al16(o + 8 * 4);
-    L.total = o;
+    L.total = (int)o;
     return L;
 }
 
@@ -230,165 +251,326 @@ __device__ __forceinline__ const float2* eig_table<true>(const DevSys& S) {
     return S.eigf;
 }
 
-// One entry of the reciprocal cluster table of branches (i, j):
-//   Z_p[s][r] = sum_{c in p} kappa_c sum_{u,t} Psi_c[u][t][s][r] e_i[u] e~'_j[t]
-__device__ __forceinline__ double2 k4_z_entry(const DevSys& S, const DevIfc& F, const double2* kap, int ch, int q0,
-                                              int ii, int i, int j, int pc, int sr) {
-    const int nb = S.nb;
+// The reciprocal cluster tables of branch i and the slots [s0, s1) of a group of bins
+// (bin_j(slot): the slot's branch j, or -1 for a slot that needs no table):
+//   Z_p[s][r] = sum_{c in p} kappa_c sum_{u,t} Psi_c[u][t][s][r] e_i[u] e~'_j[t].
+// In two steps, the clusters of a class grouped by their second atom:
+//   B_g[t][s][r] = sum_{c in g} kappa_c sum_u Psi_c[u][t][s][r] e_i[u]   (once per i)
+//   Z_p[s][r]    = sum_{g in p} sum_t e~'_j[t] B_g[t][s][r]              (per (i,j))
+// One step per (i,j) took 340 FP64 instructions and 140 loads per entry of the 58
+// quartic clusters of diamond, as much as the contraction itself on small grids; this
+// takes 24 FP64 instructions and 12 shared loads, plus the first step's share.  B is
+// kept in phase A's staging area, bgrp groups at a time (a class has at most natoms
+// groups, and bgrp is at least 17).  Ends with a barrier.
+template <typename BinJ, typename Store>
+__device__ __forceinline__ void k4_tables(const DevSys& S, const DevIfc& F, const double2* kap, double2* B, int bgrp,
+                                          int ch, int q0, int ii, int i, int s0, int s1, BinJ bin_j, Store store) {
+    const int nb = S.nb, npi = F.npi;
     const double2* ei = S.eig + (size_t)(q0 * nb + i) * nb;
-    const double2* ej = S.eig + (size_t)(ii * nb + j) * nb;
-    double2 acc = make_double2(0.0, 0.0);
-    for (int x = F.cl_start[pc]; x < F.cl_start[pc + 1]; x++) {
-        const int c = F.cl_index[x];
-        const int4 at = F.atoms[c];
-        const double* ph = F.phi + (size_t)c * 81 + sr;
-        double2 t1 = make_double2(0.0, 0.0);
+    for (int p0 = 0; p0 < npi;) {
+        const int g0 = F.cls_grp[p0];
+        int p1 = npi;
+        if (F.cls_grp[npi] - g0 > bgrp)
+            for (p1 = p0 + 1; p1 < npi && F.cls_grp[p1 + 1] - g0 <= bgrp;) p1++;
+        const int ng = F.cls_grp[p1] - g0;
+        for (int x = threadIdx.x; x < ng * 27; x += blockDim.x) {
+            const int g = x / 27, tsr = x - g * 27;
+            double2 acc = make_double2(0.0, 0.0);
+            for (int y = F.grp_start[g0 + g]; y < F.grp_start[g0 + g + 1]; y++) {
+                const int c = F.cl_index[y];
+                const double2* e = ei + 3 * F.atoms[c].x;
+                const double* f = F.phi + (size_t)c * 81 + tsr;
+                double2 t1 = make_double2(0.0, 0.0);
 #pragma unroll
-        for (int u = 0; u < 3; u++) {
-            const double2 eu = ei[3 * at.x + u];
-#pragma unroll
-            for (int t = 0; t < 3; t++) {
-                double2 et = ej[3 * at.y + t];
-                if (ch == 2) et = cconj(et);
-                const double2 pr = cmul(eu, et);
-                const double f = ph[(u * 3 + t) * 9];
-                t1.x = fma(f, pr.x, t1.x);
-                t1.y = fma(f, pr.y, t1.y);
+                for (int u = 0; u < 3; u++) {
+                    const double2 eu = e[u];
+                    const double fu = f[u * 27];
+                    t1.x = fma(fu, eu.x, t1.x);
+                    t1.y = fma(fu, eu.y, t1.y);
+                }
+                acc = cmac(acc, kap[c], t1);
             }
+            B[x] = acc;
         }
-        acc = cmac(acc, kap[c], t1);
+        __syncthreads();
+        const int n9 = (p1 - p0) * 9;
+        for (int x = threadIdx.x; x < (s1 - s0) * n9; x += blockDim.x) {
+            const int sl = x / n9, rem = x - sl * n9, pr = rem / 9, sr = rem - pr * 9;
+            const int j = bin_j(s0 + sl);
+            if (j < 0) continue;
+            const double2* ej = S.eig + (size_t)(ii * nb + j) * nb;
+            double2 acc = make_double2(0.0, 0.0);
+            for (int g = F.cls_grp[p0 + pr]; g < F.cls_grp[p0 + pr + 1]; g++) {
+                const double2* e = ej + 3 * F.grp_a2[g];
+                const double2* b = B + (g - g0) * 27 + sr;
+#pragma unroll
+                for (int t = 0; t < 3; t++) {
+                    double2 et = e[t];
+                    if (ch == 2) et = cconj(et);
+                    acc = cmac(acc, et, b[t * 9]);
+                }
+            }
+            store(s0 + sl, p0 + pr, sr, acc);
+        }
+        __syncthreads();
+        p0 = p1;
     }
-    return acc;
 }
 
-// Contract one queued process of branches (i, j) against the table Zj and add
-// its weights for every temperature to accr/accw (LIST: also store its Gamma).
-template <int NT, bool MIXED, bool LIST>
-__device__ __forceinline__ void k4_entry(const P4Params& p, const typename CT<MIXED>::T* Zj,
-                                         const typename CT<MIXED>::T* PT, const int4* blkinfo, int nbk,
-                                         unsigned long long ent, double sigma, long long pos, int ch, int ii, int i,
-                                         int j, double omega, int m0, int m1, int m2, int n0, int n1, int n2,
-                                         double (&accr)[NT], double (&accw)[NT]) {
+// Bloch phase w_p(q'') of one class: the product of the class's phase-table entries
+// of the axes along which its displacement is not a multiple of the grid (bits of fl);
+// the other factors are exactly 1.  ph: the table positions of the three coordinates
+// (a, N0 + b, N0 + N1 + c), 8 bits each.
+template <bool MIXED>
+__device__ __forceinline__ typename CT<MIXED>::T k4_class_phase(const typename CT<MIXED>::T* pt, int fl, unsigned ph) {
     using C = CT<MIXED>;
-    using cx = typename C::T;
+    const unsigned xa = ph & 0xff, xb = (ph >> 8) & 0xff, xc = ph >> 16;
+    typename C::T w;
+    if (fl & 1) {
+        w = pt[xa];
+        if (fl & 2) w = C::mul(w, pt[xb]);
+        if (fl & 4) w = C::mul(w, pt[xc]);
+    } else if (fl & 2) {
+        w = pt[xb];
+        if (fl & 4) w = C::mul(w, pt[xc]);
+    } else {
+        w = pt[xc];
+    }
+    return w;
+}
+
+// The weight of one process that all temperatures share: its Gaussian over sigma and
+// the four frequencies.  r2, r3: the (omega, Bose factors) records of the third and
+// fourth phonon.
+struct K4Weight {
+    double base;
+    const double *r2, *r3;
+};
+template <int NT>
+__device__ __forceinline__ K4Weight k4_weight(const P4Params& p, unsigned long long ent, double sigma, int ch,
+                                              const double* r1, double omega) {
     const DevSys& S = p.S;
-    const int nb = S.nb;
-    const int N0 = S.n[0], N1 = S.n[1], lsum = N0 + N1 + S.n[2];
     const double sqrtpi = sqrt(3.141592653589793238);
     const double floor_sigma = (double)0.001f;
-    const bool neg = (ch != 0);  // class displacement D = m_k - m_l (++) or m_l - m_k (+-, --)
-    const cx* etab = eig_table<MIXED>(S);
     int a, b, c, ss, k, l;
     unpack_proc(ent, a, b, c, ss, k, l);
-    const int jj = q_index(S, a, b, c);
-    // (omega, Bose factors) records of the three other modes: omega now, the factors
-    // (same cache line) after the contraction, so that they are not live across it
-    constexpr int WS = wb_stride(NT);
-    const double* x1 = p.wb + (size_t)(ii * nb + j) * WS;
-    const double* x2 = p.wb + (size_t)(jj * nb + k) * WS;
-    const double* x3 = p.wb + (size_t)(ss * nb + l) * WS;
-    const double w1 = x1[0], w2 = x2[0], w3 = x3[0];
+    K4Weight g;
+    g.r2 = p.wb + (size_t)(q_index(S, a, b, c) * S.nb + k) * wb_stride(NT);
+    g.r3 = p.wb + (size_t)(ss * S.nb + l) * wb_stride(NT);
+    const double w1 = r1[0], w2 = g.r2[0], w3 = g.r3[0];
     const double sv = (ch == 2) ? __dadd_rn(omega, -w1) : __dadd_rn(omega, w1);
     const double delta = (ch == 0) ? __dadd_rn(__dadd_rn(sv, w2), -w3) : __dadd_rn(__dadd_rn(sv, -w2), -w3);
     if (sigma <= floor_sigma) sigma = 1.0 / sqrtpi;
-    const double g = exp(-(delta * delta) / (sigma * sigma));
-    const double base = g / (sigma * sqrtpi * (omega * w1 * w2 * w3));
-    double v2 = 0.0;
-    if (LIST || !S.onlyharmonic) {
-        const cx* e2 = etab + (size_t)(jj * nb + k) * nb;
-        const cx* e3 = etab + (size_t)(ss * nb + l) * nb;
-        cx V = C::zero();
-        for (int bb = 0; bb < nbk; bb++) {
-            const int4 bi = blkinfo[bb];
-            const int p0 = bi.x, p1 = bi.y, a3 = bi.z, a4 = bi.w;
-            cx u[3], v[3];
-#pragma unroll
-            for (int x = 0; x < 3; x++) {
-                u[x] = e2[3 * a3 + x];
-                if (ch != 0) u[x] = C::conj(u[x]);
-                v[x] = C::conj(e3[3 * a4 + x]);
-            }
-            for (int pc = p0; pc < p1; pc++) {
-                const cx* pt = PT + pc * lsum;
-                cx w = C::mul(C::mul(pt[a], pt[N0 + b]), pt[N0 + N1 + c]);
-                if (neg) w = C::conj(w);
-                const cx* z = Zj + pc * 9;
-                cx tt = C::zero();
-#pragma unroll
-                for (int x = 0; x < 3; x++) {
-                    cx h = C::zero();
-#pragma unroll
-                    for (int r = 0; r < 3; r++) h = C::mac(h, z[x * 3 + r], v[r]);
-                    tt = C::mac(tt, u[x], h);
-                }
-                V = C::mac(V, w, tt);
-            }
-        }
-        v2 = C::norm(V);
-    }
-#pragma unroll
-    for (int t = 0; t < NT; t++) {
-        if (t < p.nT) {
-            const double f1 = x1[1 + t], f2 = x2[1 + t], f3 = x3[1 + t];
-            double bc;
-            if (ch == 0)
-                bc = f1 * f2 * (1 + f3) - (1 + f1) * (1 + f2) * f3;
-            else if (ch == 1)
-                bc = f1 * (1 + f2) * (1 + f3) - (1 + f1) * f2 * f3;
-            else
-                bc = (1 + f1) * (1 + f2) * (1 + f3) - f1 * f2 * f3;
-            const double wp4 = bc * base;
-            accr[t] = fma(wp4, v2, accr[t]);
-            accw[t] += wp4;
-            if (LIST) p.gamma_out[ch][pos] = wp4 * v2 * p.gamma_scale;
-        }
-    }
+    g.base = exp(-(delta * delta) / (sigma * sigma)) / (sigma * sqrtpi * (omega * w1 * w2 * w3));
+    return g;
+}
+// WP4 of the process at temperature t.
+__device__ __forceinline__ double k4_wp4(const K4Weight& g, const double* r1, int ch, int t) {
+    const double f1 = r1[1 + t], f2 = g.r2[1 + t], f3 = g.r3[1 + t];
+    double bc;
+    if (ch == 0)
+        bc = f1 * f2 * (1 + f3) - (1 + f1) * (1 + f2) * f3;
+    else if (ch == 1)
+        bc = f1 * (1 + f2) * (1 + f3) - (1 + f1) * f2 * f3;
+    else
+        bc = (1 + f1) * (1 + f2) * (1 + f3) - f1 * f2 * f3;
+    return bc * g.base;
 }
 
-// Phase B: contract every queued process of the current work item, branch by branch.
-// LIST: also store each process's own Gamma at its list position (Ind_plusplus etc.).
-template <int NT, bool MIXED, bool LIST>
-__device__ void k4_phase_b(const P4Params& p, unsigned char* smem, const Layout& L, const unsigned long long* qbase,
-                           const double* qsig, const long long* qpos, int ch, int ii, int q0, int m0, int m1, int m2,
-                           int n0, int n1, int n2, unsigned long long& my_contr) {
+// The three components of atom `a` in an eigenvector row.  FP64 rows of an even number
+// of components start on a multiple of 32 bytes, so two of the three come in one 32-byte
+// load (three 32-byte loads of a random 96-byte row take 92 SM cycles per warp, six
+// 16-byte loads 135; 55 and 81 when the rows hit L1).  FP32 rows are read component by
+// component: 16-byte pairs made the 8^3 zincblende kernel 1.5 % slower.
+__device__ __forceinline__ void load_atom(const double2* row, int a, bool even, double2 (&v)[3]) {
+    const double2* p = row + 3 * a;
+    const int one = (a & 1) ? 0 : 2;  // the component that is not in an aligned pair
+    if (even) {
+        const double2* q = p + (a & 1);
+        double2 x, y;
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x.x), "=d"(x.y), "=d"(y.x), "=d"(y.y) : "l"(q));
+        const double2 z = p[one];
+        v[0] = (a & 1) ? z : x;
+        v[1] = (a & 1) ? x : y;
+        v[2] = (a & 1) ? y : z;
+    } else {
+        v[0] = p[0];
+        v[1] = p[1];
+        v[2] = p[2];
+    }
+}
+__device__ __forceinline__ void load_atom(const float2* row, int a, bool, float2 (&v)[3]) {
+    const float2* p = row + 3 * a;
+    v[0] = p[0];
+    v[1] = p[1];
+    v[2] = p[2];
+}
+
+// |V|^2 of one queued process of bin (i, j) against its table Z (for the +- and --
+// channels Z holds the conjugate table: w, u and v are then all conjugated in V, and
+// |V|^2 is taken from its conjugate).
+//   FP64: the rows H_s = sum_{p, r} w_p Z_p[s][r] v_r of one third-phonon atom are
+//   summed over its classes first and folded with u_s once per atom, which takes 12
+//   complex multiply-adds per class instead of 13 and a phase (9 where w_p = 1), keeps
+//   the third phonon's eigenvector out of the class loop and loads it once.
+//   FP32: w_p (u Z_p v) per class.
+template <bool MIXED>
+__device__ __forceinline__ double k4_contract(const DevSys& S, const typename CT<MIXED>::T* Z,
+                                              const typename CT<MIXED>::T* PT, const unsigned char* cfl,
+                                              const int4* blkinfo, int nbk, unsigned long long ent, bool conj_v) {
     using C = CT<MIXED>;
     using cx = typename C::T;
+    const int nb = S.nb, N0 = S.n[0], N01 = N0 + S.n[1], lsum = N01 + S.n[2];
+    const bool even = (nb & 1) == 0;
+    const cx* etab = eig_table<MIXED>(S);
+    int a, b, c, ss, k, l;
+    unpack_proc(ent, a, b, c, ss, k, l);
+    const cx* row3 = etab + (q_index(S, a, b, c) * nb + k) * nb;
+    const cx* row4 = etab + (ss * nb + l) * nb;
+    const unsigned ph = a | ((N0 + b) << 8) | ((N01 + c) << 16);
+    cx V = C::zero();
+    cx H[3];  // FP64: the rows of the current third-phonon atom; FP32: its eigenvector components
+    cx v[3];
+    int a3 = -1, a4 = -1;
+    auto fold = [&]() {
+        cx u[3];
+        load_atom(row3, a3, even, u);
+#pragma unroll
+        for (int x = 0; x < 3; x++) V = C::mac(V, u[x], H[x]);
+    };
+#pragma unroll 1
+    for (int bb = 0; bb < nbk; bb++) {
+        const int4 bi = blkinfo[bb];
+        if (bi.z != a3) {
+            if (!MIXED && a3 >= 0) fold();
+            a3 = bi.z;
+            if (MIXED) {
+                load_atom(row3, a3, even, H);
+            } else {
+#pragma unroll
+                for (int x = 0; x < 3; x++) H[x] = C::zero();
+            }
+        }
+        if (bi.w != a4) {
+            a4 = bi.w;
+            load_atom(row4, a4, even, v);
+            if (conj_v) {
+#pragma unroll
+                for (int x = 0; x < 3; x++) v[x].y = -v[x].y;
+            }
+        }
+#pragma unroll 1
+        for (int pc = bi.x; pc < bi.y; pc++) {
+            const cx* z = Z + pc * 9;
+            const int fl = cfl[pc];
+            cx w;
+            if (fl) w = k4_class_phase<MIXED>(PT + pc * lsum, fl, ph);
+            cx tt = C::zero();
+#pragma unroll
+            for (int x = 0; x < 3; x++) {
+                cx h = C::zero();
+#pragma unroll
+                for (int r = 0; r < 3; r++) h = C::mac(h, z[x * 3 + r], v[r]);
+                if (MIXED) {
+                    tt = C::mac(tt, H[x], h);
+                } else if (fl) {
+                    H[x] = C::mac(H[x], w, h);
+                } else {
+                    H[x].x += h.x;
+                    H[x].y += h.y;
+                }
+            }
+            if (MIXED) {
+                if (fl) {
+                    V = C::mac(V, w, tt);
+                } else {
+                    V.x += tt.x;
+                    V.y += tt.y;
+                }
+            }
+        }
+    }
+    if (!MIXED && a3 >= 0) fold();
+    return C::norm(V);
+}
+
+// Phase B: contract every queued process of the current work item, for all (i,j)
+// bins at once when their tables fit in shared memory (L.allz), else one branch i
+// at a time.  LIST: also store each process's own Gamma at its list position
+// (Ind_plusplus etc.).
+//   The queued processes go one to a lane in bin order, across the bins: a warp sees
+// one or two bins, whose Z entries it reads as broadcasts.  Rate sums stay in registers
+// while the warp's branch i is the same and are then reduced over the warp, so that
+// one lane adds them to the work item's sums.
+// Returns the number of processes that this thread contracted.
+template <int NT, bool MIXED, bool LIST>
+__device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const double* qsig, const long long* qpos,
+                                       int ch, int ii, int q0) {
+    using C = CT<MIXED>;
+    using cx = typename C::T;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const P4Params& p = reinterpret_cast<const K4Shared*>(smem)->p;
+    const Layout& L = reinterpret_cast<const K4Shared*>(smem)->L;
+    int my_contr = 0;
     const DevSys& S = p.S;
     const DevIfc& F = p.F;
     const int nb = S.nb, nb2 = nb * nb, npi = F.npi;
     cx* Z = reinterpret_cast<cx*>(smem + L.z);
     const double2* kap = reinterpret_cast<const double2*>(smem + L.kap);
-    const cx* PT = reinterpret_cast<const cx*>(smem + L.pt);
     double* racc = reinterpret_cast<double*>(smem + L.racc);
     double* wacc = reinterpret_cast<double*>(smem + L.wacc);
-    double* red = reinterpret_cast<double*>(smem + L.red);
     int* cnt = reinterpret_cast<int*>(smem + L.cnt);
-    int* pre = reinterpret_cast<int*>(smem + L.pre);
+    int* pre = reinterpret_cast<int*>(smem + L.pre);    // entries before each bin of the group
+    const cx* PT = reinterpret_cast<const cx*>(smem + L.pt);
+    const unsigned char* cfl = smem + L.cfl;
     const int4* blkinfo = reinterpret_cast<const int4*>(smem + L.blk);
     const int nbk = reinterpret_cast<const int*>(smem + L.misc)[3];
     const double* wvw = reinterpret_cast<const double*>(S.wv) + 3;
-    for (int i = 0; i < nb; i++) {
-        if (threadIdx.x == 0) {
-            int acc = 0;
-            for (int j = 0; j < nb; j++) {
-                pre[j] = acc;
-                acc += min(cnt[i * nb + j], p.subcap);
+    const int lane = threadIdx.x & 31;
+    const bool need_v = LIST || !S.onlyharmonic;
+    const int gbins = L.allz ? nb2 : nb;
+    for (int bin0 = 0; bin0 < nb2; bin0 += gbins) {
+        if (threadIdx.x < 32) {  // prefixes of the entries over the group's bins
+            int e_run = 0;
+            unsigned branches = 0;  // branches i with entries
+            for (int b0 = 0; b0 < gbins; b0 += 32) {
+                const int b = b0 + lane;
+                const int n = b < gbins ? min(cnt[bin0 + b], p.subcap) : 0;
+                int e = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, e, o);
+                    if (lane >= o) e += y;
+                }
+                if (b < gbins) pre[b] = e_run + e - n;
+                e_run += __shfl_sync(0xffffffffu, e, 31);
+                branches |= __reduce_or_sync(0xffffffffu, n > 0 ? 1u << ((bin0 + b) / nb) : 0u);
             }
-            pre[nb] = acc;
+            if (lane == 0) {
+                pre[gbins] = e_run;
+                if (branches) atomicAdd(&p.stats[4], (unsigned long long)__popc(branches));
+            }
         }
         __syncthreads();
-        const int tot = pre[nb];
+        const int tot = pre[gbins];
         if (tot == 0) {
             __syncthreads();
             continue;
         }
-        if (threadIdx.x == 0) atomicAdd(&p.stats[4], 1ull);
-        for (int idx = threadIdx.x; idx < nb * npi * 9; idx += blockDim.x) {
-            const int j = idx / (npi * 9), rem = idx - j * (npi * 9), pc = rem / 9, sr = rem - pc * 9;
-            Z[idx] = C::from(k4_z_entry(S, F, kap, ch, q0, ii, i, j, pc, sr));
+        if (need_v) {
+            double2* B = reinterpret_cast<double2*>(smem + L.stg);
+            for (int s0 = 0; s0 < gbins; s0 += nb) {
+                if (pre[s0 + nb] == pre[s0]) continue;  // no entries of this branch
+                k4_tables(
+                    S, F, kap, B, L.bgrp, ch, q0, ii, (bin0 + s0) / nb, s0, s0 + nb,
+                    [&](int s) { return cnt[bin0 + s] > 0 ? s - s0 : -1; },
+                    [&](int s, int pc, int sr, double2 z) {
+                        if (ch != 0) z.y = -z.y;
+                        Z[(s * npi + pc) * 9 + sr] = C::from(z);
+                    });
+            }
         }
-        __syncthreads();
-        // plain per-thread partial sums (a few tens of terms each); the cross-work-item
+        // plain per-lane partial sums (a few tens of terms each); the cross-work-item
         // reduction (k4_reduce) is the compensated one
         double accr[NT], accw[NT];
 #pragma unroll
@@ -396,145 +578,94 @@ __device__ void k4_phase_b(const P4Params& p, unsigned char* smem, const Layout&
             accr[t] = 0.0;
             accw[t] = 0.0;
         }
-        const double omega = wvw[4 * (q0 * nb + i)];
-        for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-            int j = 0;
-            while (j + 1 < nb && pre[j + 1] <= e) j++;
-            const size_t qi = (size_t)(i * nb + j) * p.subcap + (e - pre[j]);
-            k4_entry<NT, MIXED, LIST>(p, Z + (size_t)j * npi * 9, PT, blkinfo, nbk, qbase[qi], qsig[qi],
-                                      LIST ? qpos[qi] : 0, ch, ii, i, j, omega, m0, m1, m2, n0, n1, n2, accr, accw);
-            my_contr++;
-        }
-        double v[2 * NT];
+        // the warp's sums of (r, w) into branch i
+        auto add_warp = [&](int i, int t, double r, double w) {
 #pragma unroll
-        for (int t = 0; t < NT; t++) {
-            v[t] = accr[t];
-            v[NT + t] = accw[t];
-        }
-        block_sum_vec<2 * NT>(v, red);
-        if (threadIdx.x == 0) {
-            for (int t = 0; t < p.nT; t++) {
-                racc[i * NT + t] += v[t];
-                wacc[i * NT + t] += v[NT + t];
+            for (int o = 16; o > 0; o >>= 1) {
+                r += __shfl_down_sync(0xffffffffu, r, o);
+                w += __shfl_down_sync(0xffffffffu, w, o);
             }
-        }
-        __syncthreads();
-    }
-    for (int x = threadIdx.x; x < nb2; x += blockDim.x) cnt[x] = 0;
-    __syncthreads();
-}
-
-// Phase B with the tables of all (i,j) in shared memory at once: one table build
-// and one pass over every queued process of the work item.  A thread's entries
-// run in (i,j) order; its sums for one branch go to shared memory when its
-// branch changes.
-template <int NT, bool MIXED, bool LIST>
-__device__ void k4_phase_b_all(const P4Params& p, unsigned char* smem, const Layout& L,
-                               const unsigned long long* qbase, const double* qsig, const long long* qpos, int ch,
-                               int ii, int q0, int m0, int m1, int m2, int n0, int n1, int n2,
-                               unsigned long long& my_contr) {
-    using C = CT<MIXED>;
-    using cx = typename C::T;
-    const DevSys& S = p.S;
-    const DevIfc& F = p.F;
-    const int nb = S.nb, nb2 = nb * nb, npi = F.npi;
-    cx* Z = reinterpret_cast<cx*>(smem + L.z);
-    const double2* kap = reinterpret_cast<const double2*>(smem + L.kap);
-    const cx* PT = reinterpret_cast<const cx*>(smem + L.pt);
-    double* racc = reinterpret_cast<double*>(smem + L.racc);
-    double* wacc = reinterpret_cast<double*>(smem + L.wacc);
-    int* cnt = reinterpret_cast<int*>(smem + L.cnt);
-    int* pre = reinterpret_cast<int*>(smem + L.pre);
-    const int4* blkinfo = reinterpret_cast<const int4*>(smem + L.blk);
-    const int nbk = reinterpret_cast<const int*>(smem + L.misc)[3];
-    const double* wvw = reinterpret_cast<const double*>(S.wv) + 3;
-    if (threadIdx.x == 0) {
-        int acc = 0, built = 0;
-        for (int i = 0; i < nb; i++) {
-            int bi = 0;
-            for (int j = 0; j < nb; j++) {
-                pre[i * nb + j] = acc;
-                const int n = min(cnt[i * nb + j], p.subcap);
-                acc += n;
-                bi += n;
+            if (lane == 0) {
+                atomicAdd(&racc[i * NT + t], r);
+                atomicAdd(&wacc[i * NT + t], w);
             }
-            built += (bi > 0);
+        };
+        int cur_i = -1, b = 0;
+        // each lane loads its next queue entry one iteration ahead
+        int b_n = 0;
+        unsigned long long ent_n;
+        double sig_n;
+        {
+            const int e = min((int)threadIdx.x, tot - 1);
+            while (pre[b_n + 1] <= e) b_n++;
+            const size_t q = (size_t)(bin0 + b_n) * p.subcap + (e - pre[b_n]);
+            ent_n = qbase[q];
+            sig_n = qsig[q];
         }
-        pre[nb2] = acc;
-        if (built) atomicAdd(&p.stats[4], (unsigned long long)built);
-    }
-    __syncthreads();
-    const int tot = pre[nb2];
-    if (tot > 0) {
-        for (int idx = threadIdx.x; idx < nb2 * npi * 9; idx += blockDim.x) {
-            const int bin = idx / (npi * 9);
-            if (cnt[bin] == 0) continue;
-            const int rem = idx - bin * (npi * 9), pc = rem / 9, sr = rem - pc * 9;
-            const int i = bin / nb, j = bin - i * nb;
-            Z[idx] = C::from(k4_z_entry(S, F, kap, ch, q0, ii, i, j, pc, sr));
-        }
-        __syncthreads();
-        double accr[NT], accw[NT];
+        for (int e0 = threadIdx.x - lane; e0 < tot; e0 += blockDim.x) {
+            const int e = min(e0 + lane, tot - 1);  // lanes past the end repeat the last entry with zero weight
+            const bool own = e0 + lane < tot;
+            b = b_n;
+            const int bin = bin0 + b, i = bin / nb, j = bin - i * nb;
+            const unsigned long long ent = ent_n;
+            const double sig = sig_n;
+            const size_t qi = (size_t)bin * p.subcap + (e - pre[b]);
+            if (e0 + (int)blockDim.x < tot) {
+                const int e2 = min(e + (int)blockDim.x, tot - 1);
+                while (pre[b_n + 1] <= e2) b_n++;
+                const size_t q = (size_t)(bin0 + b_n) * p.subcap + (e2 - pre[b_n]);
+                ent_n = qbase[q];
+                sig_n = qsig[q];
+            }
+            double v2 = 0.0;
+            K4Weight g;
+            if constexpr (MIXED) {  // the weights' loads fly during the contraction
+                g = k4_weight<NT>(p, ent, sig, ch, p.wb + (size_t)(ii * nb + j) * wb_stride(NT),
+                                  wvw[4 * (q0 * nb + i)]);
+                if (need_v) v2 = k4_contract<MIXED>(S, Z + b * npi * 9, PT, cfl, blkinfo, nbk, ent, ch == 0);
+            } else {  // they would take registers from it
+                if (need_v) v2 = k4_contract<MIXED>(S, Z + b * npi * 9, PT, cfl, blkinfo, nbk, ent, ch == 0);
+                asm volatile("" ::: "memory");
+                g = k4_weight<NT>(p, ent, sig, ch, p.wb + (size_t)(ii * nb + j) * wb_stride(NT),
+                                  wvw[4 * (q0 * nb + i)]);
+            }
+            const double* r1 = p.wb + (size_t)(ii * nb + j) * wb_stride(NT);
+            my_contr += own;
+            // one branch in the whole warp, or branches i_lo..i_hi at a boundary
+            const int i_lo = __shfl_sync(0xffffffffu, i, 0), i_hi = __shfl_sync(0xffffffffu, i, 31);
+            if (cur_i >= 0 && (cur_i != i_lo || i_lo != i_hi)) {
 #pragma unroll
-        for (int t = 0; t < NT; t++) {
-            accr[t] = 0.0;
-            accw[t] = 0.0;
-        }
-        // each thread loads its next queue entry one iteration ahead
-        int bin_n = 0, cur_i = -1;
-        double omega = 0.0;
-        unsigned long long ent_n = 0;
-        double sig_n = 0.0;
-        if ((int)threadIdx.x < tot) {
-            while (pre[bin_n + 1] <= (int)threadIdx.x) bin_n++;
-            const size_t q1 = (size_t)bin_n * p.subcap + (threadIdx.x - pre[bin_n]);
-            ent_n = qbase[q1];
-            sig_n = qsig[q1];
-        }
-        for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-            const int bin = bin_n;
-            const unsigned long long ent_c = ent_n;
-            const double sig_c = sig_n;
-            const int e2 = e + blockDim.x;
-            if (e2 < tot) {
-                while (pre[bin_n + 1] <= e2) bin_n++;
-                const size_t q2 = (size_t)bin_n * p.subcap + (e2 - pre[bin_n]);
-                ent_n = qbase[q2];
-                sig_n = qsig[q2];
+                for (int t = 0; t < NT; t++) {
+                    if (t < p.nT) add_warp(cur_i, t, accr[t], accw[t]);
+                    accr[t] = 0.0;
+                    accw[t] = 0.0;
+                }
             }
-            const int i = bin / nb, j = bin - i * nb;
-            if (i != cur_i) {
-                if (cur_i >= 0) {
+            cur_i = i_lo == i_hi ? i_lo : -1;
 #pragma unroll
-                    for (int t = 0; t < NT; t++) {
-                        if (t < p.nT) {
-                            atomicAdd(&racc[cur_i * NT + t], accr[t]);
-                            atomicAdd(&wacc[cur_i * NT + t], accw[t]);
-                        }
-                        accr[t] = 0.0;
-                        accw[t] = 0.0;
+            for (int t = 0; t < NT; t++)
+                if (t < p.nT) {
+                    const double wp4 = own ? k4_wp4(g, r1, ch, t) : 0.0;
+                    if (LIST && own) p.gamma_out[ch][qpos[qi]] = wp4 * v2 * p.gamma_scale;
+                    if (cur_i >= 0) {
+                        accr[t] = own ? fma(wp4, v2, accr[t]) : accr[t];
+                        accw[t] += wp4;
+                    } else {
+                        for (int x = i_lo; x <= i_hi; x++)
+                            add_warp(x, t, (own && i == x) ? wp4 * v2 : 0.0, (own && i == x) ? wp4 : 0.0);
                     }
                 }
-                cur_i = i;
-                omega = wvw[4 * (q0 * nb + i)];
-            }
-            const size_t qi = (size_t)bin * p.subcap + (e - pre[bin]);
-            k4_entry<NT, MIXED, LIST>(p, Z + (size_t)bin * npi * 9, PT, blkinfo, nbk, ent_c, sig_c,
-                                      LIST ? qpos[qi] : 0, ch, ii, i, j, omega, m0, m1, m2, n0, n1, n2, accr, accw);
-            my_contr++;
         }
         if (cur_i >= 0) {
 #pragma unroll
             for (int t = 0; t < NT; t++)
-                if (t < p.nT) {
-                    atomicAdd(&racc[cur_i * NT + t], accr[t]);
-                    atomicAdd(&wacc[cur_i * NT + t], accw[t]);
-                }
+                if (t < p.nT) add_warp(cur_i, t, accr[t], accw[t]);
         }
+        __syncthreads();
     }
-    __syncthreads();
     for (int x = threadIdx.x; x < nb2; x += blockDim.x) cnt[x] = 0;
     __syncthreads();
+    return my_contr;
 }
 
 // ---------------------------------------------------------------------------- tensor-core phase B
@@ -667,12 +798,16 @@ __device__ void k4_phase_b_tc(const P4Params& p, unsigned char* smem, const Layo
         if (ng == 0 || misc[7]) break;
         const long long tg0 = clock64();
         // FP64 reciprocal cluster entries of the group's bins
-        for (int idx = threadIdx.x; idx < ng * npi * 9; idx += blockDim.x) {
-            const int slot = idx / (npi * 9), rem = idx - slot * (npi * 9), pc = rem / 9, sr = rem - pc * 9;
-            const int bin = gbin[slot], i = bin / nb, j = bin - i * nb;
-            Zs[idx] = k4_z_entry(S, F, kap, ch, q0, ii, i, j, pc, sr);
+        for (int s0 = 0; s0 < ng;) {
+            const int i = gbin[s0] / nb;
+            int s1 = s0 + 1;
+            while (s1 < ng && gbin[s1] / nb == i) s1++;
+            k4_tables(
+                S, F, kap, reinterpret_cast<double2*>(smem + L.stg), L.bgrp, ch, q0, ii, i, s0, s1,
+                [&](int s) { return gbin[s] - i * nb; },
+                [&](int s, int pc, int sr, double2 z) { Zs[(s * npi + pc) * 9 + sr] = z; });
+            s0 = s1;
         }
-        __syncthreads();
         // their B tables, 16 bytes (8 values of one row n) per store
         const int chunks16 = bin_bytes >> 4;
         for (int idx = threadIdx.x; idx < ng * chunks16; idx += blockDim.x) {
@@ -860,27 +995,24 @@ __device__ void k4_phase_b_tc(const P4Params& p, unsigned char* smem, const Layo
 template <int NT, bool MIXED, bool LIST, bool TC>
 __device__ __forceinline__ void k4_flush_body(const P4Params& p, unsigned char* smem, const Layout& L,
                                               const unsigned long long* qbase, const double* qsig, const long long* qpos,
-                                              int ch, int ii, int q0, int m0, int m1, int m2, int n0, int n1, int n2,
+                                              int ch, int ii, int q0,
                                               unsigned long long& my_contr) {
     if constexpr (TC) {
         const TcPlan* P = p.tc;
         const Layout Lb = k4_layout_tcbase(NT, p.S.nb, p.F.npi, p.F.ntri, p.S.n[0] + p.S.n[1] + p.S.n[2], p.S.nptk);
         const TcLayout TL = k4_tc_layout(Lb.total, P->ksteps, P->bin_bytes, P->zbins, p.F.npi, P->chunk_cap, p.S.nb);
         k4_phase_b_tc<NT>(p, smem, L, TL, qbase, qsig, ch, ii, q0, my_contr);
-    } else if (L.allz) {
-        k4_phase_b_all<NT, MIXED, LIST>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2, my_contr);
     } else {
-        k4_phase_b<NT, MIXED, LIST>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2, my_contr);
+        my_contr += k4_phase_b<NT, MIXED, LIST>(qbase, qsig, qpos, ch, ii, q0);
     }
 }
 
 template <int NT, bool MIXED, bool LIST, bool TC>
 __device__ __forceinline__ void k4_flush(const P4Params& p, unsigned char* smem, const Layout& L,
                                          const unsigned long long* qbase, const double* qsig, const long long* qpos,
-                                         int ch, int ii, int q0, int m0, int m1, int m2, int n0, int n1, int n2,
-                                         unsigned long long& my_contr) {
+                                         int ch, int ii, int q0, unsigned long long& my_contr) {
     const long long t0 = clock64();  // thread 0 adds the CTA's cycles in phase B to stats[9]
-    k4_flush_body<NT, MIXED, LIST, TC>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2, my_contr);
+    k4_flush_body<NT, MIXED, LIST, TC>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
     if (threadIdx.x == 0) atomicAdd(&p.stats[9], (unsigned long long)(clock64() - t0));
 }
 
@@ -949,7 +1081,7 @@ __device__ void k4_list_segment(const P4Params& p, unsigned char* smem, const La
     int iter = 0;
     for (long long base = 0; base < total; base += blockDim.x, iter++) {
         if ((iter % kCheckEvery) == 0 && queue_nearly_full(p, cnt, nb2, misc))
-            k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2, my_contr);
+            k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
         const long long e = base + threadIdx.x;
         if (e >= total) continue;
         int i = 0;
@@ -992,7 +1124,7 @@ __device__ void k4_list_segment(const P4Params& p, unsigned char* smem, const La
         qpos[qi] = pos;
     }
     __syncthreads();
-    k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2, my_contr);
+    k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
 }
 
 // Per-thread work counters of one kernel, flushed into a P4Params::stats array.
@@ -1050,9 +1182,18 @@ __device__ int k4_jj_list(const DevSys& S, int ch, int jj_lo, int n0, int n1, in
     return total;
 }
 
+// The kernel's arguments and its shared-memory layout, copied for phase B.
+__device__ __forceinline__ void k4_share_args(const P4Params& p, const Layout& L, unsigned char* smem) {
+    const int* src = reinterpret_cast<const int*>(&p);
+    int* dst = reinterpret_cast<int*>(&reinterpret_cast<K4Shared*>(smem)->p);
+    for (int x = threadIdx.x; x < (int)(sizeof(P4Params) / sizeof(int)); x += blockDim.x) dst[x] = src[x];
+    if (threadIdx.x == 0) reinterpret_cast<K4Shared*>(smem)->L = L;
+    __syncthreads();
+}
+
 // Per-CTA tables of one solve: (k,l) decode table, non-empty class blocks and
 // per-class phase tables.
-template <int KIND, bool MIXED>
+template <int KIND, bool MIXED, bool TC = false>
 __device__ void k4_cta_init(const P4Params& p, unsigned char* smem, const Layout& L) {
     using C = CT<MIXED>;
     using cx = typename C::T;
@@ -1069,8 +1210,14 @@ __device__ void k4_cta_init(const P4Params& p, unsigned char* smem, const Layout
         int nbk = 0;
         if (KIND >= 2)
             for (int b = 0; b < F.nblk; b++)
-                if (F.blk_start[b] < F.blk_start[b + 1])
-                    blkinfo[nbk++] = make_int4(F.blk_start[b], F.blk_start[b + 1], b / S.natoms, b % S.natoms);
+            {
+                // FP64: the fourth-phonon atom runs back and forth, so that its eigenvector is
+                // often the one already loaded
+                const int a3 = b / S.natoms, x = b % S.natoms, a4 = (!MIXED && (a3 & 1)) ? S.natoms - 1 - x : x;
+                const int bs = a3 * S.natoms + a4;
+                if (F.blk_start[bs] < F.blk_start[bs + 1])
+                    blkinfo[nbk++] = make_int4(F.blk_start[bs], F.blk_start[bs + 1], a3, a4);
+            }
         misc[3] = nbk;
     }
     if (KIND >= 2) {
@@ -1081,6 +1228,13 @@ __device__ void k4_cta_init(const P4Params& p, unsigned char* smem, const Layout
             int4 D = F.pi_d[pc];
             int Dd = (d == 0) ? D.x : (d == 1 ? D.y : D.z);
             PT[x] = C::from(S.root[d][pmod(xi * Dd, S.n[d])]);
+        }
+        if (!TC) {
+            unsigned char* cfl = smem + L.cfl;
+            for (int pc = threadIdx.x; pc < npi; pc += blockDim.x) {
+                const int4 D = F.pi_d[pc];
+                cfl[pc] = (pmod(D.x, N0) != 0) | ((pmod(D.y, N1) != 0) << 1) | ((pmod(D.z, N2) != 0) << 2);
+            }
         }
     }
     __syncthreads();
@@ -1105,7 +1259,6 @@ __device__ __forceinline__ void k4_item(const P4Params& p, unsigned char* smem, 
     int* sidx = reinterpret_cast<int*>(smem + L.sidx);
     int* cnt = reinterpret_cast<int*>(smem + L.cnt);
     int* ncnt = reinterpret_cast<int*>(smem + L.ncnt);
-    int* klt = reinterpret_cast<int*>(smem + L.klt);
     int* misc = reinterpret_cast<int*>(smem + L.misc);
     constexpr bool LIST = (KIND == 3);
     const double sqrtpi = sqrt(3.141592653589793238);
@@ -1181,31 +1334,47 @@ __device__ __forceinline__ void k4_item(const P4Params& p, unsigned char* smem, 
         const int jj_lo = (ch == 1) ? 0 : ii;
         // the +- and -- channels walk only the q'' whose q''' is not smaller
         const bool use_list = (ch != 0) && L.njjl >= nptk;
-        const unsigned short* jjl = reinterpret_cast<const unsigned short*>(smem + L.jjl);
         const int nq = use_list ? k4_jj_list(S, ch, jj_lo, n0, n1, n2, m0, m1, m2,
                                              reinterpret_cast<unsigned short*>(smem + L.jjl),
                                              reinterpret_cast<int*>(smem + L.jjl + al16((size_t)L.njjl * 2)))
                                 : nptk - jj_lo;
         const int total = nq * nb2;
+        // Segments: phase A until a queue is nearly full or the candidates end, then phase
+        // B.  The drain is outside phase A's loop, and the loop's pointers are formed anew
+        // in each segment (the empty asm hides that they are the same), so that no value of
+        // phase A is kept across the call of phase B.
+        for (int seg = 0; seg < total;) {
+        int fresh = 0;
+        asm volatile("" : "+r"(fresh));
+        unsigned char* sm = smem + fresh;
+        const double* sval = reinterpret_cast<const double*>(sm + L.sval);
+        const double* swj = reinterpret_cast<const double*>(sm + L.swj);
+        const int* sidx = reinterpret_cast<const int*>(sm + L.sidx);
+        const int* klt = reinterpret_cast<const int*>(sm + L.klt);
+        const unsigned short* jjl = reinterpret_cast<const unsigned short*>(sm + L.jjl);
+        int* cnt = reinterpret_cast<int*>(sm + L.cnt);
+        int* ncnt = reinterpret_cast<int*>(sm + L.ncnt);
+        double* pacc = reinterpret_cast<double*>(sm + L.pacc);
+        int* misc = reinterpret_cast<int*>(sm + L.misc);
+        double4* stg = reinterpret_cast<double4*>(sm + L.stg);
+        int4* stgi = reinterpret_cast<int4*>(sm + L.stgi);
         // thread t covers index base+t; keep (jj, kl) of it incrementally
         const int Bq = blockDim.x / nb2, Br = blockDim.x % nb2;
-        int cj = threadIdx.x / nb2, ckl = threadIdx.x % nb2;
+        int cj = (seg + (int)threadIdx.x) / nb2, ckl = (seg + (int)threadIdx.x) % nb2;
         int iter = 0;
-        double4* stg = reinterpret_cast<double4*>(smem + L.stg);
-        int4* stgi = reinterpret_cast<int4*>(smem + L.stgi);
         int stage_first = 0;
-        for (int base = 0; base < total; base += blockDim.x, iter++) {
+        int base = seg;
+        seg = total;
+        for (; base < total; base += blockDim.x, iter++) {
             if ((iter % L.stgp) == 0) {
                 __syncthreads();
                 // Queue capacity: an append that leaves a bin with fewer than stgp passes
                 // of room (one entry per thread and pass) raises misc[2]; at this barrier
-                // every thread sees the flag, and the queues are drained before the next
-                // stgp passes, which cannot then overflow them.
+                // every thread sees the flag, and the segment ends: the queues are drained
+                // before the next stgp passes, which cannot then overflow them.
                 if (KIND == 2 && misc[2]) {
-                    k4_flush<NT, MIXED, LIST, TC>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2,
-                                                my_contr);
-                    __syncthreads();  // every thread has read the flag
-                    if (threadIdx.x == 0) misc[2] = 0;
+                    seg = base;
+                    break;
                 }
                 // stage the points of the next stgp passes: their records, their partners and theirs
                 stage_first = base / nb2;
@@ -1331,9 +1500,10 @@ __device__ __forceinline__ void k4_item(const P4Params& p, unsigned char* smem, 
             }
         }
         if (KIND == 2) {
-            __syncthreads();
-            k4_flush<NT, MIXED, LIST, TC>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, m0, m1, m2, n0, n1, n2,
-                                        my_contr);
+            __syncthreads();  // every thread has read the flag, every append is in place
+            if (threadIdx.x == 0) misc[2] = 0;
+            k4_flush<NT, MIXED, LIST, TC>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
+        }
         }
     }
     __syncthreads();
@@ -1362,10 +1532,12 @@ __device__ __forceinline__ void k4_item(const P4Params& p, unsigned char* smem, 
 }
 
 template <int KIND, int NT, bool MIXED>
-__global__ void __launch_bounds__(kThreads, (ctas_per_sm<KIND, NT, MIXED>())) k4_work(P4Params p) {
+__global__ void __launch_bounds__(kThreads, (ctas_per_sm<KIND, NT, MIXED>())) k4_work(const __grid_constant__ P4Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nb2 = p.S.nb * p.S.nb;
-    const Layout L = k4_layout(KIND, NT, MIXED, p.S.nb, p.F.npi, p.F.ntri, p.S.n[0] + p.S.n[1] + p.S.n[2], p.S.nptk);
+    k4_share_args(p, k4_layout(KIND, NT, MIXED, p.S.nb, p.F.npi, p.F.ntri, p.S.n[0] + p.S.n[1] + p.S.n[2], p.S.nptk),
+                  smem);
+    const Layout& L = reinterpret_cast<const K4Shared*>(smem)->L;
     int* misc = reinterpret_cast<int*>(smem + L.misc);
     k4_cta_init<KIND, MIXED>(p, smem, L);
     unsigned long long* qbase = p.queue + (size_t)blockIdx.x * nb2 * p.subcap;
@@ -1398,7 +1570,7 @@ __global__ void __launch_bounds__(kThreads, 2) k4_work_tc(P4Params p) {
     int* misc = reinterpret_cast<int*>(smem + L.misc);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TL.bar);
     uint32_t* slotw = reinterpret_cast<uint32_t*>(smem + TL.slot);
-    k4_cta_init<2, true>(p, smem, L);
+    k4_cta_init<2, true, true>(p, smem, L);
     {  // the plan, copied into shared memory
         const int* src = reinterpret_cast<const int*>(P);
         int* dst = reinterpret_cast<int*>(smem + TL.plan);
@@ -1486,13 +1658,13 @@ __global__ void __launch_bounds__(kThreads, kMultiCtasPerSm) k4_work_multi(const
                                                                                 double* queue_sigma, int cta_bins,
                                                                                 int subcap) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ P4Params sp;
+    const P4Params& sp = reinterpret_cast<const K4Shared*>(smem)->p;  // the current slot's arguments
     __shared__ int s_slot, s_wi;
     unsigned long long* qbase = queue + (size_t)blockIdx.x * cta_bins * subcap;
     double* qsig = queue_sigma + (size_t)blockIdx.x * cta_bins * subcap;
     K4Stats st{0, 0, 0, 0};
     int cur = -1;
-    Layout L{};
+    const Layout& L = reinterpret_cast<const K4Shared*>(smem)->L;
     const int total = tick->prefix[tick->nranges];
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1513,11 +1685,11 @@ __global__ void __launch_bounds__(kThreads, kMultiCtasPerSm) k4_work_multi(const
         if (slot != cur) {
             if (cur >= 0) k4_flush_stats(sp.stats, st, reinterpret_cast<double*>(smem + L.red));
             __syncthreads();
-            const int* src = reinterpret_cast<const int*>(slots + slot);
-            int* dst = reinterpret_cast<int*>(&sp);
-            for (int x = threadIdx.x; x < (int)(sizeof(P4Params) / sizeof(int)); x += blockDim.x) dst[x] = src[x];
-            __syncthreads();
-            L = k4_layout(2, NT, MIXED, sp.S.nb, sp.F.npi, sp.F.ntri, sp.S.n[0] + sp.S.n[1] + sp.S.n[2], 0, kAllZCap2);
+            const P4Params& np = slots[slot];
+            k4_share_args(np,
+                          k4_layout(2, NT, MIXED, np.S.nb, np.F.npi, np.F.ntri, np.S.n[0] + np.S.n[1] + np.S.n[2], 0,
+                                    kAllZCap2),
+                          smem);
             k4_cta_init<2, MIXED>(sp, smem, L);
             cur = slot;
         }
