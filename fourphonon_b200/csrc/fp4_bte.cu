@@ -8,7 +8,8 @@
 // each step's sum over the mode's processes across its threads (a tree
 // reduction, so only the summation order inside one step differs from the
 // reference's left-to-right loop).  F_n stays in the Fortran layout
-// F_n(nbands,nptk,3).
+// F_n(nbands,nptk,3).  The three-phonon sweep keeps the order with far less in the
+// chain (k_block_sums, k_block_steps).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -193,6 +194,212 @@ __global__ void __launch_bounds__(1024) k_sweep(BteParams p) {
             }
         }
     }
+}
+
+// The three-phonon sweep in blocks of consecutive irreducible points.  While the steps
+// of a block run, F changes only at the block's own points (the stars of its
+// irreducible points), so each step's sum splits into the terms at all other points,
+// which k_block_sums forms for every step of the block at once on the whole GPU, and
+// the few at the block's points (about 2 n B / nptk of a mode's 2 n terms for B points),
+// which it lists and k_block_steps adds in the reference's step order from shared
+// memory.  k_sweep put every term of a step into the chain: 13.5 us a step on the 12^3
+// diamond grid (140 ms a sweep).
+constexpr int kBlockPoints = 64;   // points of a block (one star may have more)
+constexpr int kStepThreads = 128;  // threads of k_block_steps
+
+struct StepInfo {
+    double base[3];  // tau v omega
+    double sum[3];   // the terms outside the block
+    double tau;
+    long long term;       // its first listed term
+    int cnt, slot, band;  // listed terms inside the block, the step's point and branch
+};
+struct BlockParams {
+    const int* step0;           // first step of each irreducible point, over the whole sweep
+    const long long* term0;     // first listed term of each mode's steps, within its block
+    int* slot_of;               // point -> its slot in the block, -1 outside
+    StepInfo* info;             // [step of the block]
+    int* idx;                   // listed terms: slot * nb + branch
+    double* coef;               //               and signed amplitude
+};
+
+// Slots of the points of the stars [l0, l1); a point met twice keeps its first slot.
+__device__ void mark_block(const BteParams& p, const BlockParams& q, int l0, int l1) {
+    int s = 0;
+    for (int ll = l0; ll < l1; ll++) {
+        for (int kk = threadIdx.x; kk < p.nequi[ll]; kk += blockDim.x)  // -1 is the largest unsigned value
+            atomicMin(reinterpret_cast<unsigned*>(q.slot_of + p.allequi[ll * p.nsr + kk] - 1), (unsigned)(s + kk));
+        s += p.nequi[ll];
+    }
+}
+
+__global__ void k_block_begin(BteParams p, BlockParams q, int l1) {
+    for (int x = threadIdx.x; x < p.nptk; x += blockDim.x) q.slot_of[x] = -1;
+    __syncthreads();
+    mark_block(p, q, 0, l1);
+}
+
+// One CTA per step of the block [l0, l1).
+__global__ void __launch_bounds__(256) k_block_sums(BteParams p, BlockParams q, int l0, int l1) {
+    __shared__ double red[3][32];
+    __shared__ int s_cnt;
+    const int nb = p.nb;
+    const int step = q.step0[l0] + blockIdx.x;
+    int ll = l0;
+    while (q.step0[ll + 1] <= step) ll++;
+    const int neq = p.nequi[ll], rest = step - q.step0[ll], i = rest / neq, kk = rest - i * neq;
+    const int mm = ll * nb + i;
+    const int qq = p.allequi[ll * p.nsr + kk] - 1, sym = p.typeofsym[ll * p.nsr + kk] - 1;
+    const int np_ = p.n_plus[mm], nt = np_ + p.n_minus[mm];
+    const long long op = p.off_plus[mm], om = p.off_minus[mm];
+    const long long out = q.term0[mm] + (long long)kk * 2 * nt;
+    const int lim = p.nptk * nb;
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    double a[3] = {0.0, 0.0, 0.0};
+    const size_t pl = (size_t)lim;
+    auto term = [&](int b, int qx, double g) {  // g F(b, qx), or its entry in the list
+        const int slot = q.slot_of[qx];
+        if (slot >= 0) {
+            const int pos = atomicAdd(&s_cnt, 1);  // at most 2 nt terms
+            q.idx[out + pos] = slot * nb + b;
+            q.coef[out + pos] = g;
+        } else {
+            const double* f = p.F + (size_t)qx * nb + b;
+            a[0] = fma(g, f[0], a[0]);
+            a[1] = fma(g, f[pl], a[1]);
+            a[2] = fma(g, f[2 * pl], a[2]);
+        }
+    };
+    for (int x = threadIdx.x; x < nt; x += blockDim.x) {
+        const bool plus = x < np_;
+        const long long o = plus ? op + x : om + (x - np_);
+        const int x2 = (plus ? p.i2p : p.i2m)[o] - 1, x3 = (plus ? p.i3p : p.i3m)[o] - 1;
+        if (x2 < 0 || x2 >= lim || x3 < 0 || x3 >= lim) {
+            atomicOr(p.err, kErrList);
+            continue;
+        }
+        const int m2 = x2 / nb, n3 = x3 / nb;
+        const double g = plus ? p.gp[o] : p.gm[o] * 5.e-1;
+        term(x3 - n3 * nb, p.id_equi[(size_t)n3 * p.nsr + sym] - 1, g);
+        term(x2 - m2 * nb, p.id_equi[(size_t)m2 * p.nsr + sym] - 1, plus ? -g : g);
+    }
+    block_sum3(a[0], a[1], a[2], red);  // its barrier also ends the appends
+    if (threadIdx.x == 0) {
+        const double tz = p.tau_zero[mm];
+        const size_t e = (size_t)i * p.nptk + qq;
+        const double w = p.energy[e];
+        StepInfo s;
+        for (int d = 0; d < 3; d++) {
+            s.base[d] = tz * p.velocity[e + d * pl] * w;
+            s.sum[d] = a[d];
+        }
+        s.tau = tz;
+        s.term = out;
+        s.cnt = s_cnt;
+        s.slot = q.slot_of[qq];
+        s.band = i;
+        q.info[blockIdx.x] = s;
+    }
+}
+
+// The block's steps in order, on one CTA; then the marks of the next block [l1, l2).
+// Shared memory: F and the symmetrizer of each of the block's npts points.
+__global__ void __launch_bounds__(kStepThreads) k_block_steps(BteParams p, BlockParams q, int l0, int l1, int l2,
+                                                              int npts) {
+    extern __shared__ double sm[];
+    __shared__ double red[3][kStepThreads / 32];
+    const int nb = p.nb, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* Fs = sm;                        // [slot][band][3]
+    double* Ss = sm + (size_t)npts * nb * 3;  // [slot][9]
+    int s0 = 0;
+    for (int ll = l0; ll < l1; ll++) {
+        const int neq = p.nequi[ll];
+        for (int x = threadIdx.x; x < neq * nb; x += blockDim.x) {
+            const int kk = x / nb, b = x - kk * nb, qq = p.allequi[ll * p.nsr + kk] - 1;
+            for (int d = 0; d < 3; d++) Fs[((s0 + kk) * nb + b) * 3 + d] = Fat(p, b, qq, d);
+        }
+        for (int x = threadIdx.x; x < neq * 9; x += blockDim.x)
+            Ss[s0 * 9 + x] = p.symm[9 * (size_t)(p.allequi[ll * p.nsr + x / 9] - 1) + x % 9];
+        s0 += neq;
+    }
+    __syncthreads();
+    // a step's record is read two steps ahead, each thread's first two of its terms one
+    // step ahead: no load of the chain's own step is waited for
+    const int nsteps = q.step0[l1] - q.step0[l0];
+    auto record = [&](int st) { return q.info[min(st, nsteps - 1)]; };
+    auto terms = [&](const StepInfo& s, int (&ix)[2], double (&cf)[2]) {
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+            const int x = threadIdx.x + y * kStepThreads;
+            ix[y] = x < s.cnt ? q.idx[s.term + x] : 0;
+            cf[y] = x < s.cnt ? q.coef[s.term + x] : 0.0;
+        }
+    };
+    StepInfo s_1{}, s_2{};
+    int ix_1[2] = {0, 0};
+    double cf_1[2] = {0.0, 0.0};
+    if (nsteps > 0) {
+        s_1 = record(0);
+        s_2 = record(1);
+        terms(s_1, ix_1, cf_1);
+    }
+    for (int st = 0; st < nsteps; st++) {
+        const StepInfo s = s_1;
+        const int ix[2] = {ix_1[0], ix_1[1]};
+        const double cf[2] = {cf_1[0], cf_1[1]};
+        s_1 = s_2;
+        s_2 = record(st + 2);
+        terms(s_1, ix_1, cf_1);
+        double a[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int y = 0; y < 2; y++)
+            if (threadIdx.x + y * kStepThreads < s.cnt)
+                for (int d = 0; d < 3; d++) a[d] = fma(cf[y], Fs[ix[y] * 3 + d], a[d]);
+        for (int x = threadIdx.x + 2 * kStepThreads; x < s.cnt; x += kStepThreads) {
+            const int ii = q.idx[s.term + x];
+            const double g = q.coef[s.term + x];
+            for (int d = 0; d < 3; d++) a[d] = fma(g, Fs[ii * 3 + d], a[d]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int d = 0; d < 3; d++) a[d] += __shfl_down_sync(0xffffffffu, a[d], o);
+        if (lane == 0)
+            for (int d = 0; d < 3; d++) red[d][warp] = a[d];
+        __syncthreads();
+        // the step's branch takes its new value, then F_n(:,qq,:) is symmetrised
+        if (threadIdx.x < nb) {
+            double* f = Fs + (s.slot * nb + threadIdx.x) * 3;
+            double y[3] = {f[0], f[1], f[2]};
+            if (threadIdx.x == s.band) {
+                for (int d = 0; d < 3; d++) {
+                    double in = 0.0;
+#pragma unroll
+                    for (int w = 0; w < kStepThreads / 32; w++) in += red[d][w];
+                    y[d] = s.base[d] + s.tau * (s.sum[d] + in);
+                }
+            }
+            const double* Sq = Ss + s.slot * 9;
+            for (int d = 0; d < 3; d++) f[d] = Sq[d] * y[0] + Sq[d + 3] * y[1] + Sq[d + 6] * y[2];
+        }
+        __syncthreads();
+    }
+    s0 = 0;
+    for (int l = l0; l < l1; l++) {
+        const int neq = p.nequi[l];
+        for (int x = threadIdx.x; x < neq * nb; x += blockDim.x) {
+            const int k = x / nb, b = x - k * nb, qq = p.allequi[l * p.nsr + k] - 1;
+            if (q.slot_of[qq] != s0 + k) continue;  // a repeated point lives in its first slot
+            for (int d = 0; d < 3; d++) Fat(p, b, qq, d) = Fs[((s0 + k) * nb + b) * 3 + d];
+        }
+        s0 += neq;
+    }
+    __syncthreads();
+    for (int l = l0; l < l1; l++)
+        for (int k = threadIdx.x; k < p.nequi[l]; k += blockDim.x) q.slot_of[p.allequi[l * p.nsr + k] - 1] = -1;
+    __syncthreads();
+    mark_block(p, q, l1, l2);
 }
 
 // The Jacobi form of the same update (no counterpart in the reference, whose
@@ -418,6 +625,46 @@ struct Lists4 {
 };
 }  // namespace
 
+static size_t block_smem(int nb, int pts) { return (size_t)pts * (nb * 3 + 9) * sizeof(double); }
+
+// Cuts the irreducible points into blocks of at most kBlockPoints points (or one star),
+// and lays out their steps and, for the worst case that every term falls inside the
+// block, their listed terms; terms, steps and pts are the largest block's.  False when a
+// block's terms or points would take too much memory: the sweep then runs on k_sweep.
+static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* n_plus, const int32_t* n_minus,
+                        std::vector<int>& cut, std::vector<int>& step0, std::vector<long long>& term0, size_t& terms,
+                        size_t& steps, int& pts) {
+    const size_t kMaxTerms = (size_t)32 << 20;  // 384 MB of indices and amplitudes
+    const size_t kMaxSmem = 200 * 1024;
+    cut.assign(1, 0);
+    step0.assign(nlist + 1, 0);
+    term0.assign((size_t)nb * nlist, 0);
+    terms = steps = 0;
+    pts = 0;
+    size_t bt = 0;
+    int bp = 0;
+    for (int ll = 0; ll < nlist; ll++) {
+        size_t lt = 0;
+        for (int i = 0; i < nb; i++) lt += (size_t)2 * ((size_t)n_plus[ll * nb + i] + n_minus[ll * nb + i]) * nequi[ll];
+        if (ll > cut.back() && (bp + nequi[ll] > kBlockPoints || bt + lt > kMaxTerms)) {
+            cut.push_back(ll);
+            bt = 0;
+            bp = 0;
+        }
+        for (int i = 0; i < nb; i++) {
+            term0[(size_t)ll * nb + i] = (long long)bt;
+            bt += (size_t)2 * ((size_t)n_plus[ll * nb + i] + n_minus[ll * nb + i]) * nequi[ll];
+        }
+        bp += nequi[ll];
+        step0[ll + 1] = step0[ll] + nb * nequi[ll];
+        terms = std::max(terms, bt);
+        steps = std::max(steps, (size_t)(step0[ll + 1] - step0[cut.back()]));
+        pts = std::max(pts, bp);
+    }
+    cut.push_back(nlist);
+    return terms <= kMaxTerms && block_smem(nb, pts) <= kMaxSmem;
+}
+
 static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int32_t* nequi, const int32_t* allequi,
                      const int32_t* typeofsym, int32_t nsr, const int32_t* id_equi, const double* symmetrizers,
                      const int32_t* n_plus, const int32_t* n_minus, int32_t ntotal_plus, int32_t ntotal_minus,
@@ -572,12 +819,58 @@ static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int3
         CK(cudaMemcpyAsync(f_n, Fout, (size_t)nptk * nb * 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         return fp4_end(c);
     }
-    CK(cudaEventRecord(c->evk0, c->stream));
-    k_sweep<<<1, 1024, 0, c->stream>>>(p);
-    CK(cudaGetLastError());
-    CK(cudaEventRecord(c->evk1, c->stream));
+    std::vector<int> cut;  // blocks [cut[x], cut[x+1]) of irreducible points
+    std::vector<int> step0;
+    std::vector<long long> term0;
+    size_t terms = 0, steps = 0;
+    int pts = 0;
+    const bool blocks = !l4 && plan_blocks(nb, nlist, nequi, n_plus, n_minus, cut, step0, term0, terms, steps, pts);
+    if (blocks) {
+        // [slot_of | step0] and [term0], [records], [idx], [coef] in one buffer
+        auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        const size_t o1 = up((size_t)nptk * sizeof(int)), o2 = o1 + up((nlist + 1) * sizeof(int)),
+                     o3 = o2 + up(nm * sizeof(long long)), o4 = o3 + up(steps * sizeof(StepInfo)),
+                     o5 = o4 + up(terms * sizeof(double)), o6 = o5 + up(terms * sizeof(int));
+        if ((r = B[12].reserve(c, o6))) return r;
+        unsigned char* d = B[12].as<unsigned char>();
+        BlockParams q{};
+        q.slot_of = reinterpret_cast<int*>(d);
+        q.step0 = reinterpret_cast<const int*>(d + o1);
+        q.term0 = reinterpret_cast<const long long*>(d + o2);
+        q.info = reinterpret_cast<StepInfo*>(d + o3);
+        q.coef = reinterpret_cast<double*>(d + o4);
+        q.idx = reinterpret_cast<int*>(d + o5);
+        CK(cudaMemcpyAsync(d + o1, step0.data(), (nlist + 1) * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(d + o2, term0.data(), nm * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+        const size_t smem = block_smem(nb, pts);
+        CK(cudaFuncSetAttribute(k_block_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaEventRecord(c->evk0, c->stream));
+        k_block_begin<<<1, 1024, 0, c->stream>>>(p, q, cut[1]);
+        CK(cudaGetLastError());
+        c->launches++;
+        for (size_t x = 0; x + 1 < cut.size(); x++) {
+            const int l0 = cut[x], l1 = cut[x + 1], l2 = x + 2 < cut.size() ? cut[x + 2] : l1;
+            const int ns = step0[l1] - step0[l0];
+            if (ns) {
+                k_block_sums<<<ns, 256, 0, c->stream>>>(p, q, l0, l1);
+                CK(cudaGetLastError());
+                c->launches++;
+            }
+            int np = 0;
+            for (int ll = l0; ll < l1; ll++) np += nequi[ll];
+            k_block_steps<<<1, kStepThreads, smem, c->stream>>>(p, q, l0, l1, l2, np);
+            CK(cudaGetLastError());
+            c->launches++;
+        }
+        CK(cudaEventRecord(c->evk1, c->stream));
+    } else {
+        CK(cudaEventRecord(c->evk0, c->stream));
+        k_sweep<<<1, 1024, 0, c->stream>>>(p);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(c->evk1, c->stream));
+        c->launches++;
+    }
     c->kernel_timed = true;
-    c->launches++;
     CK(cudaMemcpyAsync(f_n, B[5].ptr, (size_t)nptk * nb * 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     B[5].key = 0;  // device copy now differs from the caller's previous F_n
     return fp4_end(c);
