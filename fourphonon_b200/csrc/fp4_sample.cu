@@ -10,10 +10,10 @@
 // the CPU oracle draws exactly the same samples.
 //
 // One CTA takes a chunk of samples of one (mode, channel): its threads draw
-// and filter, survivors go to a shared-memory list, and then each thread
-// contracts one survivor's V(4) directly over the clusters (phases from the
-// integer lattice coordinates, as in the rate kernel).  Per-chunk sums go to a
-// buffer reduced afterwards in a fixed order with compensated sums.
+// and filter, survivors go to a shared-memory list, and the listed processes'
+// V(4) are contracted directly over the clusters (phases from the integer lattice
+// coordinates, as in the rate kernel), in FP64 by eight lanes per process.  Per-chunk
+// sums go to a buffer reduced afterwards in a fixed order with compensated sums.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -30,7 +30,10 @@ using namespace fp4;
 namespace {
 
 constexpr int kSThreads = 256;
-constexpr int kSChunk = 1024;  // samples per CTA item (= survivor list capacity)
+constexpr int kSChunk = 1024;      // fewest samples of an item
+constexpr int kSChunkMax = 16384;  // and most: about 1 % of the draws survive, so that a list fills the CTA
+constexpr int kSRounds = 2;        // rounds of one draw per thread between looks at the list
+constexpr int kSList = 1024;       // list capacity; emptied when fewer than kSRounds rounds fit
 
 struct PSParams {
     DevSys S;
@@ -39,7 +42,9 @@ struct PSParams {
     const double* bose;  // [t][q*nb+b]
     long long nsamples;
     unsigned long long seed;
+    int chunk;   // samples per item
     int nchunk;  // chunks per (mode, channel)
+    int a_tab;   // 1: the clusters contracted with the mode's eigenvector fit in shared memory
     int mode;    // 0: counts and P4, 2: rates and WP4
     int nitems;
     int* work_counter;
@@ -59,56 +64,65 @@ __device__ __forceinline__ int draw_k(unsigned long long base, int k, int range)
     return (int)__umul64hi(mix64(base + (unsigned long long)k), (unsigned long long)range);
 }
 
-// V(4) of one process, summed over the clusters (Vp_pp/pm/mm, processes.f90:142-330):
+// The terms c = c0, c0 + dc, ... of one process's V(4), summed over the clusters
+// (Vp_pp/pm/mm, processes.f90:142-330):
 //   sum_c mu_c exp(2 pi i (s_j n'.m_j + s_k n''.m_k - n'''.m_l)/N)
-//         sum_{u,t,s,r} Psi_c[u][t][s][r] e_i[u] e~'_j[t] e~''_k[s] conj(e'''_l[r])
-__device__ double2 vp4_direct(const DevSys& S, const DevIfc& F, int ch, const double2* ei, const double2* ej,
-                              const double2* ek, const double2* el, int m0, int m1, int m2, int a0, int a1, int a2,
-                              int t0, int t1, int t2) {
+//         sum_{t,s,r} A_c[t][s][r] e~'_j[t] e~''_k[s] conj(e'''_l[r]),
+// A_c[t][s][r] = sum_u Psi_c[u][t][s][r] e_i[u], from the table A of the item's mode or
+// (A == nullptr) formed here.
+__device__ double2 vp4_terms(const DevSys& S, const DevIfc& F, const double2* A, int ch, const double2* ei,
+                             const double2* ej, const double2* ek, const double2* el, int m0, int m1, int m2, int a0,
+                             int a1, int a2, int t0, int t1, int t2, int c0, int dc) {
     const int sj = (ch == 2) ? -1 : 1, sk = (ch == 0) ? 1 : -1;
     double2 V = make_double2(0.0, 0.0);
-    for (int c = 0; c < F.ntri; c++) {
+    for (int c = c0; c < F.ntri; c += dc) {
         const int4 at = F.atoms[c];
         const int4 mj = F.mj[c], mk = F.mk[c], ml = F.ml[c];
         const double2 ph =
             cmul(cmul(S.root[0][pmod(sj * m0 * mj.x + sk * a0 * mk.x - t0 * ml.x, S.n[0])],
                       S.root[1][pmod(sj * m1 * mj.y + sk * a1 * mk.y - t1 * ml.y, S.n[1])]),
                  S.root[2][pmod(sj * m2 * mj.z + sk * a2 * mk.z - t2 * ml.z, S.n[2])]);
-        double2 I[3], J[3], K[3], L[3];
+        double2 K[3], L[3];
 #pragma unroll
         for (int x = 0; x < 3; x++) {
-            I[x] = ei[3 * at.x + x];
-            J[x] = ej[3 * at.y + x];
-            if (ch == 2) J[x] = cconj(J[x]);
             K[x] = ek[3 * at.z + x];
             if (ch != 0) K[x] = cconj(K[x]);
             L[x] = cconj(el[3 * at.w + x]);
         }
         const double* psi = F.phi + (size_t)c * 81;
-        double2 A = make_double2(0.0, 0.0);
+        const double2* Ac = A ? A + (size_t)c * 27 : nullptr;
+        double2 B = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int t = 0; t < 3; t++) {
+            double2 J = ej[3 * at.y + t];
+            if (ch == 2) J = cconj(J);
+            double2 y = make_double2(0.0, 0.0);
 #pragma unroll
-        for (int u = 0; u < 3; u++) {
-            double2 wu = make_double2(0.0, 0.0);
+            for (int s = 0; s < 3; s++) {
+                double2 xs = make_double2(0.0, 0.0);
 #pragma unroll
-            for (int t = 0; t < 3; t++) {
-                double2 y = make_double2(0.0, 0.0);
+                for (int r = 0; r < 3; r++) {
+                    const int o = (t * 3 + s) * 3 + r;
+                    double2 f;
+                    if (A) {
+                        f = Ac[o];
+                    } else {
+                        f = make_double2(0.0, 0.0);
 #pragma unroll
-                for (int s = 0; s < 3; s++) {
-                    const double* row = psi + ((u * 3 + t) * 3 + s) * 3;
-                    double2 xs = make_double2(0.0, 0.0);
-#pragma unroll
-                    for (int r = 0; r < 3; r++) {
-                        xs.x = fma(row[r], L[r].x, xs.x);
-                        xs.y = fma(row[r], L[r].y, xs.y);
+                        for (int u = 0; u < 3; u++) {
+                            const double2 e = ei[3 * at.x + u];
+                            f.x = fma(psi[u * 27 + o], e.x, f.x);
+                            f.y = fma(psi[u * 27 + o], e.y, f.y);
+                        }
                     }
-                    y = cmac(y, xs, K[s]);
+                    xs = cmac(xs, f, L[r]);
                 }
-                wu = cmac(wu, y, J[t]);
+                y = cmac(y, xs, K[s]);
             }
-            A = cmac(A, wu, I[u]);
+            B = cmac(B, y, J);
         }
         const double2 w = make_double2(F.mu[c] * ph.x, F.mu[c] * ph.y);
-        V = cmac(V, w, A);
+        V = cmac(V, w, B);
     }
     return V;
 }
@@ -172,16 +186,28 @@ struct SEntry {
     double sigma, delta;
 };
 
+// Draws of one item, then V(4) and the weights of the draws that survived.  About one
+// draw in a hundred does, so that an item of 1024 draws kept ten threads of 256 walking
+// the clusters while the others waited (10 % issue activity, 15 of 18 stall cycles at a
+// barrier).  An item holds up to kSChunkMax draws instead, and in FP64 eight lanes share
+// a process's clusters; lane x of the eight then weighs temperature x.  FP32 (mixed
+// precision) keeps one lane per process, whose sum runs over the clusters in order.
+// 1.3e8 draws of the 12^3 zincblende grid at four temperatures: 52.2 ms before, 5.4 ms
+// after (4.9 ms of it here).
 template <int NT, bool MIXED>
-__global__ void __launch_bounds__(kSThreads) k4_sample(PSParams p) {
-    __shared__ SEntry q[kSChunk];
+__global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
+    extern __shared__ __align__(16) unsigned char smem_s[];
     __shared__ int s_cnt, s_item;
     __shared__ double red[32 * (2 * NT + 2)];
+    SEntry* q = reinterpret_cast<SEntry*>(smem_s);
+    double2* A = reinterpret_cast<double2*>(smem_s + kSList * sizeof(SEntry));
     const DevSys& S = p.S;
     const int nb = S.nb, nptk = S.nptk;
     const int N0 = S.n[0], N1 = S.n[1], N2 = S.n[2];
     const double sqrtpi = sqrt(3.141592653589793238);
     const double floor_sigma = (double)0.001f;
+    const bool need_v = p.mode == 2 && !S.onlyharmonic;
+    const int lane = threadIdx.x & 31, l8 = lane & 7;
     for (;;) {
         if (threadIdx.x == 0) {
             s_item = atomicAdd(p.work_counter, 1);
@@ -197,16 +223,36 @@ __global__ void __launch_bounds__(kSThreads) k4_sample(PSParams p) {
         q_coords_t(S, q0, n0, n1, n2);
         const double omega = S.wv[q0 * nb + i].w;
         const bool active = (omega != 0.0) && (omega <= S.omega_max);
-        const long long c0 = (long long)chunk * kSChunk;
-        const long long c1 = min(c0 + (long long)kSChunk, p.nsamples);
+        const long long c0 = (long long)chunk * p.chunk;
+        const long long c1 = min(c0 + (long long)p.chunk, p.nsamples);
+        const double2* ei = S.eig + (size_t)(q0 * nb + i) * nb;
         unsigned long long my_n = 0;
         Comp accP = {0.0, 0.0};
-        if (active) {
-            for (long long it = c0 + threadIdx.x; it < c1; it += blockDim.x) {
+        double acc[2 * NT];  // FP32: every temperature; FP64: [0] and [NT] of temperature l8
+#pragma unroll
+        for (int x = 0; x < 2 * NT; x++) acc[x] = 0.0;
+        if (!MIXED && need_v && p.a_tab && active) {  // A_c[t][s][r] of the item's mode
+            for (int x = threadIdx.x; x < p.F.ntri * 27; x += blockDim.x) {
+                const int c = x / 27, o = x - c * 27;
+                const double* f = p.F.phi + (size_t)c * 81 + o;
+                const double2* e = ei + 3 * p.F.atoms[c].x;
+                double2 a = make_double2(0.0, 0.0);
+#pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    a.x = fma(f[u * 27], e[u].x, a.x);
+                    a.y = fma(f[u * 27], e[u].y, a.y);
+                }
+                A[x] = a;
+            }
+        }
+        for (long long base = c0; active && base < c1;) {
+            for (int rd = 0; rd < kSRounds && base < c1; rd++, base += blockDim.x) {
+                const long long it = base + threadIdx.x;
+                if (it >= c1) continue;
                 const unsigned long long c = ((unsigned long long)((mm - 1) * 3 + ch) << 32) | (unsigned long long)it;
-                const unsigned long long base = mix64(p.seed ^ mix64(c));
-                const int ii = draw_k(base, 0, nptk), j = draw_k(base, 1, nb);
-                const int jj = draw_k(base, 2, nptk), k = draw_k(base, 3, nb), l = draw_k(base, 4, nb);
+                const unsigned long long key = mix64(p.seed ^ mix64(c));
+                const int ii = draw_k(key, 0, nptk), j = draw_k(key, 1, nb);
+                const int jj = draw_k(key, 2, nptk), k = draw_k(key, 3, nb), l = draw_k(key, 4, nb);
                 int m0c, m1c, m2c, a, b, cc;
                 q_coords_t(S, ii, m0c, m1c, m2c);
                 q_coords_t(S, jj, a, b, cc);
@@ -246,7 +292,7 @@ __global__ void __launch_bounds__(kSThreads) k4_sample(PSParams p) {
                              (sg * sqrtpi * ((double)nptk * (double)nptk * (double)nptk) * (double)(nb * nb * nb * nb)));
                     continue;
                 }
-                const int pos = atomicAdd(&s_cnt, 1);  // one survivor at most per sample: pos < kSChunk
+                const int pos = atomicAdd(&s_cnt, 1);  // kSRounds more per thread fit (below)
                 SEntry e;
                 e.ii = ii;
                 e.jj = jj;
@@ -256,21 +302,23 @@ __global__ void __launch_bounds__(kSThreads) k4_sample(PSParams p) {
                 e.delta = delta;
                 q[pos] = e;
             }
-        }
-        __syncthreads();
-        double acc[2 * NT];
-#pragma unroll
-        for (int x = 0; x < 2 * NT; x++) acc[x] = 0.0;
-        if (p.mode == 2) {
+            if (p.mode != 2) continue;
+            __syncthreads();
             const int nq = s_cnt;
-            const double2* ei = S.eig + (size_t)(q0 * nb + i) * nb;
+            if (base < c1 && nq + kSRounds * (int)blockDim.x <= kSList) {
+                __syncthreads();  // every thread has read the count
+                continue;
+            }
             const size_t plane = (size_t)nptk * nb;
-            for (int e = threadIdx.x; e < nq; e += blockDim.x) {
-                const SEntry en = q[e];
+            const int per = MIXED ? 32 : 4;  // processes of one warp at a time
+            for (int e0 = (threadIdx.x >> 5) * per; e0 < nq; e0 += (kSThreads / 32) * per) {
+                const int e = e0 + (MIXED ? lane : lane >> 3);
+                const bool own = e < nq;
+                const SEntry en = q[min(e, nq - 1)];
                 const int j = en.jkl & 0xff, k = (en.jkl >> 8) & 0xff, l = en.jkl >> 16;
                 const double w1 = S.wv[en.ii * nb + j].w, w2 = S.wv[en.jj * nb + k].w, w3 = S.wv[en.ss * nb + l].w;
                 double v2 = 0.0;
-                if (!S.onlyharmonic) {
+                if (need_v) {
                     int m0c, m1c, m2c, a, b, cc, t0, t1, t2;
                     q_coords_t(S, en.ii, m0c, m1c, m2c);
                     q_coords_t(S, en.jj, a, b, cc);
@@ -283,18 +331,26 @@ __global__ void __launch_bounds__(kSThreads) k4_sample(PSParams p) {
                                                       cc, t0, t1, t2);
                         v2 = (double)V.x * (double)V.x + (double)V.y * (double)V.y;
                     } else {
-                        const double2 V = vp4_direct(S, p.F, ch, ei, S.eig + (size_t)(en.ii * nb + j) * nb,
-                                                     S.eig + (size_t)(en.jj * nb + k) * nb,
-                                                     S.eig + (size_t)(en.ss * nb + l) * nb, m0c, m1c, m2c, a, b, cc,
-                                                     t0, t1, t2);
+                        double2 V = vp4_terms(S, p.F, p.a_tab ? A : nullptr, ch, ei,
+                                              S.eig + (size_t)(en.ii * nb + j) * nb,
+                                              S.eig + (size_t)(en.jj * nb + k) * nb,
+                                              S.eig + (size_t)(en.ss * nb + l) * nb, m0c, m1c, m2c, a, b, cc, t0, t1,
+                                              t2, l8, 8);
+                        __syncwarp();
+#pragma unroll
+                        for (int o = 4; o > 0; o >>= 1) {
+                            V.x += __shfl_xor_sync(0xffffffffu, V.x, o);
+                            V.y += __shfl_xor_sync(0xffffffffu, V.y, o);
+                        }
                         v2 = V.x * V.x + V.y * V.y;
                     }
                 }
                 const double g = exp(-(en.delta * en.delta) / (en.sigma * en.sigma));
                 const bool low = (w1 <= 1.25 || w2 <= 1.25 || w3 <= 1.25);
 #pragma unroll
-                for (int t = 0; t < NT; t++) {
-                    if (t < p.nT) {
+                for (int x = 0; x < (MIXED ? NT : 1); x++) {
+                    const int t = MIXED ? x : l8;
+                    if (own && t < p.nT) {
                         const double* bz = p.bose + t * plane;
                         const double f1 = bz[en.ii * nb + j], f2 = bz[en.jj * nb + k], f3 = bz[en.ss * nb + l];
                         double bc;
@@ -305,28 +361,36 @@ __global__ void __launch_bounds__(kSThreads) k4_sample(PSParams p) {
                         else
                             bc = (1 + f1) * (1 + f2) * (1 + f3) - f1 * f2 * f3;
                         const double wp4 = low ? 0.0 : bc * g / en.sigma / sqrtpi / (omega * w1 * w2 * w3);
-                        acc[t] = fma(wp4, v2, acc[t]);
-                        acc[NT + t] += wp4;
+                        acc[x] = fma(wp4, v2, acc[x]);
+                        acc[NT + x] += wp4;
                     }
                 }
             }
-        } else {
-            acc[0] = accP.val();
+            __syncthreads();  // the list is read
+            if (threadIdx.x == 0) s_cnt = 0;
+            __syncthreads();
         }
         double v[2 * NT + 2];
 #pragma unroll
-        for (int x = 0; x < 2 * NT; x++) v[x] = acc[x];
+        for (int x = 0; x < NT; x++) {
+            const bool mine = MIXED || p.mode != 2 || l8 == x;
+            v[x] = mine ? acc[(MIXED ? x : 0)] : 0.0;
+            v[NT + x] = mine ? acc[NT + (MIXED ? x : 0)] : 0.0;
+        }
+        if (p.mode != 2) v[0] = accP.val();
         v[2 * NT] = (double)my_n;
         v[2 * NT + 1] = 0.0;
         block_sum_vec<2 * NT + 2>(v, red);
         if (threadIdx.x == 0) {
-            for (int x = 0; x < 2 * p.nT; x++) {
-                const int src = (x < p.nT) ? x : NT + (x - p.nT);
-                p.part[(size_t)item * 2 * p.nT + x] = v[src];
-            }
+#pragma unroll
+            for (int x = 0; x < NT; x++)
+                if (x < p.nT) {
+                    p.part[(size_t)item * 2 * p.nT + x] = v[x];
+                    p.part[(size_t)item * 2 * p.nT + p.nT + x] = v[NT + x];
+                }
             p.part_n[item] = (unsigned long long)v[2 * NT];
             atomicAdd(&p.stats[0], (unsigned long long)v[2 * NT]);
-            if (p.mode == 2 && !S.onlyharmonic) atomicAdd(&p.stats[1], (unsigned long long)v[2 * NT]);
+            if (need_v) atomicAdd(&p.stats[1], (unsigned long long)v[2 * NT]);
         }
         __syncthreads();
     }
@@ -556,9 +620,15 @@ static int run_sample(fp4_ctx* c, int mode, int nT, const double* temps, int64_t
     if (mode == 2 && (nT < 1 || nT > kMaxTemps)) return fp4_fail(c, FP4_E_ARG, "nT=%d outside [1,%d]", nT, kMaxTemps);
     const DevSys& S = c->S;
     const int nm = S.nb * S.nlist;
-    const int64_t nchunk = (nsamples + kSChunk - 1) / kSChunk;
+    const int64_t smallest = (int64_t)nm * 3 * ((nsamples + kSChunk - 1) / kSChunk);
+    if (smallest > ((int64_t)1 << 30))
+        return fp4_fail(c, FP4_E_CAPACITY, "too many sample chunks (%lld)", (long long)smallest);
+    // Samples per item: large enough that an item's survivors fill its CTA, small enough
+    // that every SM gets at least eight items.
+    const int64_t per_sm = (int64_t)nm * 3 * nsamples / ((int64_t)c->sm_count * 8);
+    const int chunk = (int)std::max<int64_t>(kSChunk, std::min<int64_t>(kSChunkMax, per_sm / kSChunk * kSChunk));
+    const int64_t nchunk = (nsamples + chunk - 1) / chunk;
     const int64_t nitems = (int64_t)nm * 3 * nchunk;
-    if (nitems > ((int64_t)1 << 30)) return fp4_fail(c, FP4_E_CAPACITY, "too many sample chunks (%lld)", (long long)nitems);
     const int nt = (mode == 2) ? nT : 1;
     int r;
     if (mode == 2) {
@@ -578,6 +648,7 @@ static int run_sample(fp4_ctx* c, int mode, int nT, const double* temps, int64_t
     p.bose = mode == 2 ? c->b_bose.as<double>() : nullptr;
     p.nsamples = nsamples;
     p.seed = seed;
+    p.chunk = chunk;
     p.nchunk = (int)nchunk;
     p.mode = mode;
     p.nitems = (int)nitems;
@@ -590,11 +661,16 @@ static int run_sample(fp4_ctx* c, int mode, int nT, const double* temps, int64_t
     CK(cudaEventRecord(c->evk0, c->stream));
     // mixed precision: the V(4) sums in FP32 (the draws, filter, weights and sums stay FP64)
     const bool mixed = mode == 2 && c->precision != FP4_PREC_FP64;
-#define FP4_KS(NTV)                                                   \
-    if (mixed)                                                        \
-        k4_sample<NTV, true><<<nblocks, kSThreads, 0, c->stream>>>(p); \
-    else                                                              \
-        k4_sample<NTV, false><<<nblocks, kSThreads, 0, c->stream>>>(p);
+    size_t smem = mode == 2 ? kSList * sizeof(SEntry) : 0;
+    const size_t a_bytes = (size_t)p.F.ntri * 27 * sizeof(double2);
+    p.a_tab = mode == 2 && !mixed && !S.onlyharmonic && smem + a_bytes <= 200 * 1024;
+    if (p.a_tab) smem += a_bytes;
+#define FP4_KS(NTV)                                                                                                \
+    {                                                                                                              \
+        auto kernel = mixed ? k4_sample<NTV, true> : k4_sample<NTV, false>;                                        \
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                  \
+        kernel<<<nblocks, kSThreads, smem, c->stream>>>(p);                                                        \
+    }
     if (mode == 2 && nt > 4) {
         FP4_KS(8)
     } else if (mode == 2 && nt > 2) {
