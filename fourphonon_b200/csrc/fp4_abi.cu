@@ -396,6 +396,25 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
         if ((r = T.cls_grp.upload(c, cls_grp.data(), cls_grp.size() * sizeof(int)))) return r;
         if ((r = T.grp_start.upload(c, grp_start.data(), grp_start.size() * sizeof(int)))) return r;
         if ((r = T.grp_a2.upload(c, grp_a2.data(), grp_a2.size() * sizeof(int)))) return r;
+        // phase tables exp(2 pi i x D_d / N_d), x in [0, N_d), of the axes where D_d is not a multiple of N_d
+        std::vector<int4> cls_ph(npi);
+        std::vector<int> pt_root;
+        for (int q = 0; q < npi; q++) {
+            const int D[3] = {pi_d[q].x, pi_d[q].y, pi_d[q].z};
+            int place[3] = {0, 0, 0}, axes = 0;
+            for (int d = 0; d < 3; d++) {
+                const int N = g->ngrid[d], m = ((D[d] % N) + N) % N;
+                if (m == 0) continue;
+                axes |= 1 << d;
+                place[d] = (int)pt_root.size();
+                for (int x = 0; x < N; x++) pt_root.push_back((d << 16) | (x * m % N));
+            }
+            cls_ph[q] = make_int4(place[0], place[1], place[2], axes);
+        }
+        T.F.npt = (int)pt_root.size();
+        pt_root.push_back(0);  // never empty
+        if ((r = T.cls_ph.upload(c, cls_ph.data(), cls_ph.size() * sizeof(int4)))) return r;
+        if ((r = T.pt_root.upload(c, pt_root.data(), pt_root.size() * sizeof(int)))) return r;
     }
     T.h_blk_start = blk_start;
     DevIfc& F = T.F;
@@ -414,6 +433,8 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
     F.cls_grp = T.cls_grp.as<int>();
     F.grp_start = T.grp_start.as<int>();
     F.grp_a2 = T.grp_a2.as<int>();
+    F.cls_ph = T.cls_ph.as<int4>();
+    F.pt_root = T.pt_root.as<int>();
     F.pi_d = T.pi_d.as<int4>();
     F.blk_start = T.blk_start.as<int>();
     return FP4_OK;

@@ -41,12 +41,12 @@ struct DevBuffer {
 };
 
 struct IfcTables {
-    DevBuffer phi, atoms, mj, mk, ml, mu, cl_start, cl_index, pi_d, blk_start, cls_grp, grp_start, grp_a2;
+    DevBuffer phi, atoms, mj, mk, ml, mu, cl_start, cl_index, pi_d, blk_start, cls_grp, grp_start, grp_a2, cls_ph, pt_root;
     fp4::DevIfc F{};
     std::vector<int> h_blk_start;  // host copy of the classes' block ranges
     std::vector<DevBuffer*> list() {
-        return {&phi,      &atoms, &mj,        &mk,      &ml,        &mu,     &cl_start,
-                &cl_index, &pi_d,  &blk_start, &cls_grp, &grp_start, &grp_a2};
+        return {&phi,  &atoms,     &mj,      &mk,        &ml,     &mu,     &cl_start, &cl_index,
+                &pi_d, &blk_start, &cls_grp, &grp_start, &grp_a2, &cls_ph, &pt_root};
     }
 };
 

@@ -37,6 +37,7 @@ struct DevSys {
 
 struct DevIfc {
     int order, ntri, npi, nblk;  // nblk = natoms^2 atom-pair blocks of the class table
+    int npt;                     // 4ph: entries of the classes' phase tables
     const double* phi;           // per cluster 27 (3ph: [t][s][r]) or 81 (4ph: [u][t][s][r]) entries
     const int4* atoms;           // 0-based (a1,a2,a3,a4)
     const int4* mj;              // lattice coordinates of the 2nd atom's cell
@@ -48,6 +49,8 @@ struct DevIfc {
     const int* cls_grp;          // 4ph: class p's clusters in groups of one second atom, groups [cls_grp[p], cls_grp[p+1])
     const int* grp_start;        // 4ph: group g owns cl_index[grp_start[g] .. grp_start[g+1])
     const int* grp_a2;           // 4ph: second atom of group g
+    const int4* cls_ph;          // 4ph: places of class p's three per-axis phase tables, and (w) the axes that have one
+    const int* pt_root;          // 4ph: root of each phase-table entry, axis << 16 | power
     const int4* pi_d;            // class displacement D (x,y,z) and packed atom pair in .w
     const int* blk_start;        // classes sorted by atom-pair block: block b owns [blk_start[b], blk_start[b+1])
 };
@@ -198,29 +201,6 @@ struct Comp {
     }
     __device__ __forceinline__ double val() const { return s + c; }
 };
-
-// First index i with a[i] >= x in a sorted a[0..n-1], by a descent over powers of two
-// from the largest one <= n: the step count depends only on n, so the lanes of a warp
-// stay together.
-__device__ __forceinline__ int lower_bound_desc(const double* a, int n, double x) {
-    int i = 0;
-    if (n <= 0) return 0;
-    for (int step = 1 << (31 - __clz(n)); step > 0; step >>= 1) {
-        const int y = i + step;
-        if (y <= n && a[y - 1] < x) i = y;
-    }
-    return i;
-}
-// First index i with a[i] > x (the count of entries <= x), by the same descent.
-__device__ __forceinline__ int upper_bound_desc(const double* a, int n, double x) {
-    int i = 0;
-    if (n <= 0) return 0;
-    for (int step = 1 << (31 - __clz(n)); step > 0; step >>= 1) {
-        const int y = i + step;
-        if (y <= n && a[y - 1] <= x) i = y;
-    }
-    return i;
-}
 
 // ---------------------------------------------------------------------------
 // Energy-conservation filter, bit-exact with the reference's source order.
