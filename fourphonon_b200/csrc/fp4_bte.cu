@@ -203,7 +203,8 @@ __global__ void __launch_bounds__(1024) k_sweep(BteParams p) {
 // the few at the block's points (about 2 n B / nptk of a mode's 2 n terms for B points),
 // which it lists and k_block_steps adds in the reference's step order from shared
 // memory.  k_sweep put every term of a step into the chain: 13.5 us a step on the 12^3
-// diamond grid (140 ms a sweep).
+// diamond grid (140 ms a sweep).  Here a step of the chain is two barriers and a few
+// hundred terms; the sweep, its symmetrisation and kappa take 17.6 ms with their copies.
 constexpr int kBlockPoints = 64;   // points of a block (one star may have more)
 constexpr int kStepThreads = 128;  // threads of k_block_steps
 
@@ -737,16 +738,14 @@ static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int3
         return r;
     int* L = B[10].as<int>();
     double* G = B[11].as<double>();
-    if (tp) {
-        CK(cudaMemcpyAsync(L, i2p, tp * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(L + tp, i3p, tp * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(G, gp, tp * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    }
-    if (tm) {
-        CK(cudaMemcpyAsync(L + 2 * tp, i2m, tm * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(L + 2 * tp + tm, i3m, tm * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(G + tp, gm, tm * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    }
+    auto host = [](const void* x) { return const_cast<void*>(x); };
+    const HostCopy in[6] = {{host(i2p), L, tp * sizeof(int)},
+                            {host(i3p), L + tp, tp * sizeof(int)},
+                            {host(gp), G, tp * sizeof(double)},
+                            {host(i2m), L + 2 * tp, tm * sizeof(int)},
+                            {host(i3m), L + 2 * tp + tm, tm * sizeof(int)},
+                            {host(gm), G + tp, tm * sizeof(double)}};
+    if ((r = fp4_copy_lists(c, in, 6, false))) return r;
     BteParams p{};
     p.nb = nb;
     p.nptk = nptk;

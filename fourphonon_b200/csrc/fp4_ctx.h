@@ -69,6 +69,7 @@ struct fp4_ctx {
     DevBuffer b_energy, b_velocity, b_wv, b_eigraw, b_eig, b_eigf, b_list, b_qc, b_root[3], b_rootf[3];
     DevBuffer b_temps, b_bose, b_wb, b_out, b_out4, b_lists, b_gamma, b_off, b_counts;
     DevBuffer b_queue, b_part, b_work, b_err, b_stats;
+    unsigned char* staging = nullptr;  // pinned staging of fp4_copy_lists
     DevBuffer b_tcplan, b_wtab;  // tensor-core contraction: its plan and phase rows
     bool last_tc = false;        // the last four-phonon RTA call ran its contraction on the tensor cores
     DevBuffer b_bte[13];  // [12]: the new iterate of a Jacobi sweep
@@ -94,6 +95,16 @@ struct fp4_ctx {
         return v;
     }
 };
+
+// One copy between pageable host memory and the device.
+struct HostCopy {
+    void* host;
+    void* dev;
+    size_t bytes;
+};
+// Copies in stream order, all to the host or all to the device.  Large ones go through the
+// context's pinned buffer with several host threads; they are done when the call returns.
+int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host);
 
 int fp4_fail(fp4_ctx* c, int code, const char* fmt, ...);
 int fp4_begin(fp4_ctx* c);
