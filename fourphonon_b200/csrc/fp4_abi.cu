@@ -495,15 +495,14 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
         std::vector<int> pt_root;
         for (int q = 0; q < npi; q++) {
             const int D[3] = {pi_d[q].x, pi_d[q].y, pi_d[q].z};
-            int place[3] = {0, 0, 0}, axes = 0;
+            int place[3] = {0, 0, 0}, ntab = 0;
             for (int d = 0; d < 3; d++) {
                 const int N = g->ngrid[d], m = ((D[d] % N) + N) % N;
                 if (m == 0) continue;
-                axes |= 1 << d;
-                place[d] = (int)pt_root.size();
+                place[ntab++] = (int)pt_root.size() | (8 * d) << 24;
                 for (int x = 0; x < N; x++) pt_root.push_back((d << 16) | (x * m % N));
             }
-            cls_ph[q] = make_int4(place[0], place[1], place[2], axes);
+            cls_ph[q] = make_int4(place[0], place[1], place[2], ntab);
         }
         T.F.npt = (int)pt_root.size();
         pt_root.push_back(0);  // never empty

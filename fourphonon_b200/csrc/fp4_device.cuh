@@ -49,7 +49,7 @@ struct DevIfc {
     const int* cls_grp;          // 4ph: class p's clusters in groups of one second atom, groups [cls_grp[p], cls_grp[p+1])
     const int* grp_start;        // 4ph: group g owns cl_index[grp_start[g] .. grp_start[g+1])
     const int* grp_a2;           // 4ph: second atom of group g
-    const int4* cls_ph;          // 4ph: places of class p's three per-axis phase tables, and (w) the axes that have one
+    const int4* cls_ph;          // 4ph: class p's phase tables: (w) how many, then their places | (8 * axis) << 24
     const int* pt_root;          // 4ph: root of each phase-table entry, axis << 16 | power
     const int4* pi_d;            // class displacement D (x,y,z) and packed atom pair in .w
     const int* blk_start;        // classes sorted by atom-pair block: block b owns [blk_start[b], blk_start[b+1])

@@ -328,25 +328,18 @@ __device__ __forceinline__ void k4_tables(const DevSys& S, const DevIfc& F, cons
     }
 }
 
-// Bloch phase w_p(q'') of one class at grid point (a, b, c): the product of its phase
-// tables of the axes along which its displacement is not a multiple of the grid (bits of
-// cph.w; their places in PT are cph.x, y, z); the other factors are exactly 1.  ph: the
-// three coordinates, 8 bits each.
+// Bloch phase w_p(q'') of one class: the product of its cp.w phase-table entries
+// (DevIfc::cls_ph), the other axes' factors being exactly 1.  ph: the grid coordinates
+// of q'', 8 bits each.
 template <bool MIXED>
-__device__ __forceinline__ typename CT<MIXED>::T k4_class_phase(const typename CT<MIXED>::T* PT, int4 cph,
+__device__ __forceinline__ typename CT<MIXED>::T k4_class_phase(const typename CT<MIXED>::T* PT, int4 cp,
                                                                 unsigned ph) {
     using C = CT<MIXED>;
-    const unsigned xa = cph.x + (ph & 0xff), xb = cph.y + ((ph >> 8) & 0xff), xc = cph.z + (ph >> 16);
-    typename C::T w;
-    if (cph.w & 1) {
-        w = PT[xa];
-        if (cph.w & 2) w = C::mul(w, PT[xb]);
-        if (cph.w & 4) w = C::mul(w, PT[xc]);
-    } else if (cph.w & 2) {
-        w = PT[xb];
-        if (cph.w & 4) w = C::mul(w, PT[xc]);
-    } else {
-        w = PT[xc];
+    auto at = [&](int f) { return PT[(f & 0xffffff) + ((ph >> (f >> 24)) & 0xff)]; };
+    typename C::T w = at(cp.x);
+    if (cp.w > 1) {
+        w = C::mul(w, at(cp.y));
+        if (cp.w > 2) w = C::mul(w, at(cp.z));
     }
     return w;
 }
@@ -479,31 +472,37 @@ __device__ __forceinline__ double k4_contract(const DevSys& S, const typename CT
         for (int pc = bi.x; pc < bi.y; pc++) {
             const cx* z = Z + pc * 9;
             const int4 cp = cph[pc];
-            const int fl = cp.w;
-            cx w;
-            if (fl) w = k4_class_phase<MIXED>(PT, cp, ph);
-            cx tt = C::zero();
+            if constexpr (MIXED) {
+                cx w;
+                if (cp.w) w = k4_class_phase<MIXED>(PT, cp, ph);
+                cx tt = C::zero();
 #pragma unroll
-            for (int x = 0; x < 3; x++) {
-                cx h = C::zero();
+                for (int x = 0; x < 3; x++) {
+                    cx h = C::zero();
 #pragma unroll
-                for (int r = 0; r < 3; r++) h = C::mac(h, z[x * 3 + r], v[r]);
-                if (MIXED) {
+                    for (int r = 0; r < 3; r++) h = C::mac(h, z[x * 3 + r], v[r]);
                     tt = C::mac(tt, H[x], h);
-                } else if (fl) {
-                    H[x] = C::mac(H[x], w, h);
-                } else {
-                    H[x].x += h.x;
-                    H[x].y += h.y;
                 }
-            }
-            if (MIXED) {
-                if (fl) {
+                if (cp.w) {
                     V = C::mac(V, w, tt);
                 } else {
                     V.x += tt.x;
                     V.y += tt.y;
                 }
+            } else if (cp.w) {
+                const cx w = k4_class_phase<MIXED>(PT, cp, ph);
+#pragma unroll
+                for (int x = 0; x < 3; x++) {
+                    cx h = C::zero();
+#pragma unroll
+                    for (int r = 0; r < 3; r++) h = C::mac(h, z[x * 3 + r], v[r]);
+                    H[x] = C::mac(H[x], w, h);
+                }
+            } else {  // w = 1: straight into the rows
+#pragma unroll
+                for (int x = 0; x < 3; x++)
+#pragma unroll
+                    for (int r = 0; r < 3; r++) H[x] = C::mac(H[x], z[x * 3 + r], v[r]);
             }
         }
     }
@@ -542,8 +541,9 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
     const int4* cph = reinterpret_cast<const int4*>(smem + L.cph);
     const int4* blkinfo = reinterpret_cast<const int4*>(smem + L.blk);
     const int nbk = reinterpret_cast<const int*>(smem + L.misc)[3];
+    const int* klt = reinterpret_cast<const int*>(smem + L.klt);  // bin -> i << 8 | j
     const double* wvw = reinterpret_cast<const double*>(S.wv) + 3;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, nT = p.nT;
     const bool need_v = LIST || !S.onlyharmonic;
     const int gbins = L.allz ? nb2 : nb;
     for (int bin0 = 0; bin0 < nb2; bin0 += gbins) {
@@ -623,7 +623,7 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
             const int e = min(e0 + lane, tot - 1);  // lanes past the end repeat the last entry with zero weight
             const bool own = e0 + lane < tot;
             b = b_n;
-            const int bin = bin0 + b, i = bin / nb, j = bin - i * nb;
+            const int bin = bin0 + b, ij = klt[bin], i = ij >> 8, j = ij & 0xff;
             const unsigned long long ent = ent_n;
             const double sig = sig_n;
             const size_t qi = (size_t)bin * p.subcap + (e - pre[b]);
@@ -642,41 +642,52 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
                 if (need_v) v2 = k4_contract<MIXED>(S, Z + b * npi * 9, PT, cph, blkinfo, nbk, ent, ch == 0);
             } else {  // they would take registers from it
                 if (need_v) v2 = k4_contract<MIXED>(S, Z + b * npi * 9, PT, cph, blkinfo, nbk, ent, ch == 0);
-                asm volatile("" ::: "memory");
-                g = k4_weight<NT>(p, ent, sig, ch, p.wb + (size_t)(ii * nb + j) * wb_stride(NT),
+                unsigned long long after = ent;  // (the empty asm makes the weights wait for v2)
+                asm volatile("" : "+l"(after) : "d"(v2));
+                g = k4_weight<NT>(p, after, sig, ch, p.wb + (size_t)(ii * nb + j) * wb_stride(NT),
                                   wvw[4 * (q0 * nb + i)]);
             }
             const double* r1 = p.wb + (size_t)(ii * nb + j) * wb_stride(NT);
             my_contr += own;
-            // one branch in the whole warp, or branches i_lo..i_hi at a boundary
-            const int i_lo = __shfl_sync(0xffffffffu, i, 0), i_hi = __shfl_sync(0xffffffffu, i, 31);
-            if (cur_i >= 0 && (cur_i != i_lo || i_lo != i_hi)) {
+            // the warp's branch, or branches i_lo..i_hi where the warp meets a boundary
+            if (!__all_sync(0xffffffffu, i == cur_i)) {
+                const int i_lo = __shfl_sync(0xffffffffu, i, 0), i_hi = __shfl_sync(0xffffffffu, i, 31);
+                if (cur_i >= 0) {
 #pragma unroll
-                for (int t = 0; t < NT; t++) {
-                    if (t < p.nT) add_warp(cur_i, t, accr[t], accw[t]);
-                    accr[t] = 0.0;
-                    accw[t] = 0.0;
-                }
-            }
-            cur_i = i_lo == i_hi ? i_lo : -1;
-#pragma unroll
-            for (int t = 0; t < NT; t++)
-                if (t < p.nT) {
-                    const double wp4 = own ? k4_wp4(g, r1, ch, t) : 0.0;
-                    if (LIST && own) p.gamma_out[ch][qpos[qi]] = wp4 * v2 * p.gamma_scale;
-                    if (cur_i >= 0) {
-                        accr[t] = own ? fma(wp4, v2, accr[t]) : accr[t];
-                        accw[t] += wp4;
-                    } else {
-                        for (int x = i_lo; x <= i_hi; x++)
-                            add_warp(x, t, (own && i == x) ? wp4 * v2 : 0.0, (own && i == x) ? wp4 : 0.0);
+                    for (int t = 0; t < NT; t++) {
+                        if (NT <= 2 || t < nT) add_warp(cur_i, t, accr[t], accw[t]);
+                        accr[t] = 0.0;
+                        accw[t] = 0.0;
                     }
                 }
+                cur_i = i_lo == i_hi ? i_lo : -1;
+                if (cur_i < 0) {
+#pragma unroll
+                    for (int t = 0; t < NT; t++)
+                        if (NT <= 2 || t < nT) {
+                            const double wp4 = own ? k4_wp4(g, r1, ch, t) : 0.0;
+                            if (LIST && own) p.gamma_out[ch][qpos[qi]] = wp4 * v2 * p.gamma_scale;
+                            for (int x = i_lo; x <= i_hi; x++)
+                                add_warp(x, t, (own && i == x) ? wp4 * v2 : 0.0, (own && i == x) ? wp4 : 0.0);
+                        }
+                    continue;
+                }
+            }
+            if (own) {
+#pragma unroll
+                for (int t = 0; t < NT; t++)
+                    if (NT <= 2 || t < nT) {
+                        const double wp4 = k4_wp4(g, r1, ch, t);
+                        if (LIST) p.gamma_out[ch][qpos[qi]] = wp4 * v2 * p.gamma_scale;
+                        accr[t] = fma(wp4, v2, accr[t]);
+                        accw[t] += wp4;
+                    }
+            }
         }
         if (cur_i >= 0) {
 #pragma unroll
             for (int t = 0; t < NT; t++)
-                if (t < p.nT) add_warp(cur_i, t, accr[t], accw[t]);
+                if (NT <= 2 || t < nT) add_warp(cur_i, t, accr[t], accw[t]);
         }
         __syncthreads();
     }
