@@ -22,7 +22,7 @@
 // a fixed order with compensated summation (k4_reduce).
 //
 // What bounds it (12^3 diamond, FP64, two temperatures; 1.09 s before phase B's tables,
-// loads and sums were rearranged, 1.02 s after): no single unit.  Builds that leave one
+// loads and sums were rearranged, 0.93 s now): no single unit.  Builds that leave one
 // part out put the class loop at 40 % of phase B, the gathers of the two eigenvector
 // rows at 16 %, the weights at 16 %, the tables at 5 %.  On 8^3 the load pipe is 61 %
 // busy, FP64 28 %, issue 45 %; the top stalls are fixed latency and loads.  More warps
@@ -158,8 +158,6 @@ __host__ __device__ inline Layout k4_layout_z(int kind, int NT, bool mixed, int 
     const size_t ncopy = (kind == 0) ? (L.priv ? kThreads : kThreads / 32) : 1;
     L.pacc = (int)o;
     o = al16(o + (size_t)nb * ncopy * 8);
-    L.red = (int)o;  // block_sum_vec of the 4 work counters
-    o = al16(o + (size_t)32 * 4 * 8);
     L.cell = (int)o;  // phase A: number of sorted sums below each cell of their range
     o = al16(o + (size_t)(kCells + 2) * 2);
     L.sidx = (int)o;
@@ -183,6 +181,7 @@ __host__ __device__ inline Layout k4_layout_z(int kind, int NT, bool mixed, int 
     L.stgp = stage_passes((int)nb2);
     L.stg = (int)o;  // per staged point: the records (v, omega) of its nb branches, then those of its partner
     o = al16(o + (size_t)stage_slots((int)nb2) * 2 * nb * 32);
+    L.red = L.stg;  // the sums of the work counters, after the last work item
     L.bgrp = stage_slots((int)nb2) * 2 * nb * 32 / (27 * 16);  // cluster groups that fit there in phase B
     L.stgi = (int)o;  // per staged point: (its index, its grid coordinates packed, the partner's index)
     o = al16(o + (size_t)stage_slots((int)nb2) * 16);
@@ -217,7 +216,7 @@ __host__ __device__ inline Layout k4_layout(int kind, int NT, bool mixed, int nb
 // of one group of bins, two mbarriers, the TMEM address and the parities of the
 // two mbarriers, the group's bins and its chunk list.
 struct TcLayout {
-    size_t a, b, zs, eig, plan, bar, slot, gbin, chunk, total;
+    size_t a, b, zs, eig, plan, cls, bar, slot, gbin, chunk, total;
 };
 
 __host__ __device__ inline Layout k4_layout_tcbase(int NT, int nb, int npi, int ntri, int npt, int nptk) {
@@ -239,6 +238,8 @@ __host__ __device__ inline TcLayout k4_tc_layout(size_t base, int ksteps, int bi
     o += (size_t)2 * kTcRows * (2 * nb + 1) * 8;
     T.plan = o;  // a copy of the plan
     o = al16(o + sizeof(TcPlan));
+    T.cls = o;  // per class: its pass << 16 | its block within the pass
+    o = al16(o + (size_t)npi * 4);
     T.bar = o;
     o += 16;
     T.slot = o;
@@ -697,34 +698,31 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
 }
 
 // ---------------------------------------------------------------------------- tensor-core phase B
-// 16 bytes (8 bf16 values, k = kb..kb+7) of row n of pass `pass` of a bin's B
-// table: n runs over the pass's blocks (32 columns each: re(Z[sr]) at sr,
-// im(Z[sr]) at 9+sr) and k over its classes (6 values each, see TcPlan); zero
-// outside the class's own block.
-__device__ __forceinline__ uint4 tc_b_chunk(const TcPlan* P, const double2* Zs, int npi, int slot, int pass, int n,
-                                            int kb) {
-    const int lb = n >> 5, nn = n & 31;
-    const int4 bk = P->blk[P->pass_blk0[pass] + lb];
-    const int c0 = P->pass_cls0[pass];
-    const int cls_lo = c0 + kb / 6, cls_hi = c0 + (kb + 7) / 6;
-    uint32_t w4[4] = {0, 0, 0, 0};
-    if (nn < 18 && cls_hi >= bk.x && cls_lo < bk.y) {
-        const int ro = nn >= 9, sr = nn - 9 * ro;
+// The bf16 hi/lo values of Z_p[s][r] in a bin's B table: row n of the class's pass runs
+// over the pass's blocks (32 rows each: re(Z[sr]) at sr, im(Z[sr]) at 9+sr) and k over its
+// classes (6 values each, see TcPlan).  Everything outside a class's own block is zero in
+// every bin, so the zeros are written once per CTA (k4_work_tc) and a group of bins
+// writes its values only: three 4-byte words per (class, row) in place of every 16-byte
+// word of the table (one in seven of its entries is not zero on diamond; 7^3 diamond, two
+// temperatures: 26.6 -> 23.5 ms a call).  cls: the
+// class's pass and its block within the pass.
+__device__ __forceinline__ void tc_b_values(const TcPlan* P, unsigned char* bin, int pc, int cls, int nn, double2 z) {
+    const int pass = cls >> 16, lb = cls & 0xffff, ro = nn >= 9;
+    const int N = 32 * (P->pass_blk0[pass + 1] - P->pass_blk0[pass]);
+    const int n = lb * 32 + nn, k0 = 6 * (pc - P->pass_cls0[pass]);
+    // the product's real (ro = 0) or imaginary (ro = 1) part takes, from A's (re, im)
+    // pair of w: (Z.re, -Z.im) or (Z.im, Z.re)
+    uint16_t rh, rl, ih, il;
+    tc::split_bf16(ro ? z.y : z.x, rh, rl);
+    tc::split_bf16(ro ? z.x : -z.y, ih, il);
+    const uint32_t hi = (uint32_t)rh | (uint32_t)ih << 16, lo = (uint32_t)rl | (uint32_t)il << 16;
+    unsigned char* row = bin + P->pass_boff[pass] + (n >> 3) * 256 + (n & 7) * 16;
 #pragma unroll
-        for (int y = 0; y < 8; y++) {
-            const int k = kb + y, cls = c0 + k / 6;
-            if (cls < bk.x || cls >= bk.y) continue;
-            const int r6 = k - (k / 6) * 6, split = r6 >> 1, ri = r6 & 1;
-            const double2 z = Zs[((size_t)slot * npi + cls) * 9 + sr];
-            // the product's real (ro = 0) or imaginary (ro = 1) part takes, from A's
-            // (re, im) pair of w: (Z.re, -Z.im) or (Z.im, Z.re)
-            const double v = (ri == 0) ? (ro == 0 ? z.x : z.y) : (ro == 0 ? -z.y : z.x);
-            uint16_t hi, lo;
-            tc::split_bf16(v, hi, lo);
-            w4[y >> 1] |= (uint32_t)(split == 1 ? lo : hi) << (16 * (y & 1));
-        }
+    for (int sp = 0; sp < 3; sp++) {  // k is even: a pair never leaves its 16-byte word
+        const int k = k0 + 2 * sp;
+        *reinterpret_cast<uint32_t*>(row + (k >> 4) * (N * 32) + ((k >> 3) & 1) * 128 + (k & 7) * 2) =
+            (sp == 1) ? lo : hi;
     }
-    return make_uint4(w4[0], w4[1], w4[2], w4[3]);
 }
 
 // Phase B on the tensor cores (mixed precision, RTA): the queued processes of
@@ -762,6 +760,7 @@ __device__ void k4_phase_b_tc(const P4Params& p, unsigned char* smem, const Layo
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TL.bar);
     uint32_t* slotw = reinterpret_cast<uint32_t*>(smem + TL.slot);  // [0] TMEM base, [1+g] parity of mbarrier g
     int* gbin = reinterpret_cast<int*>(smem + TL.gbin);
+    const int* tcls = reinterpret_cast<const int*>(smem + TL.cls);
     int* chunks = reinterpret_cast<int*>(smem + TL.chunk);
     const int zbins = P->zbins, npass = P->npass, ksteps = P->ksteps, bin_bytes = P->bin_bytes;
     const int wg = threadIdx.x >> 7, m = threadIdx.x & 127, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -836,19 +835,11 @@ __device__ void k4_phase_b_tc(const P4Params& p, unsigned char* smem, const Layo
                 [&](int s, int pc, int sr, double2 z) { Zs[(s * npi + pc) * 9 + sr] = z; });
             s0 = s1;
         }
-        // their B tables, 16 bytes (8 values of one row n) per store
-        const int chunks16 = bin_bytes >> 4;
-        for (int idx = threadIdx.x; idx < ng * chunks16; idx += blockDim.x) {
-            const int slot = idx / chunks16;
-            const int off = (idx - slot * chunks16) << 4;
-            int pass = 0;
-            while (pass + 1 < npass && P->pass_boff[pass + 1] <= off) pass++;
-            const int rel = off - P->pass_boff[pass];
-            const int N = 32 * (P->pass_blk0[pass + 1] - P->pass_blk0[pass]);
-            const int s = rel / (N * 32), within = rel - s * (N * 32);
-            const int n = (within >> 8) * 8 + ((within >> 4) & 7);
-            const int kb = s * 16 + ((within >> 7) & 1) * 8;
-            *reinterpret_cast<uint4*>(Bbuf + (size_t)slot * bin_bytes + off) = tc_b_chunk(P, Zs, npi, slot, pass, n, kb);
+        // their values in the B tables
+        for (int idx = threadIdx.x; idx < ng * npi * 18; idx += blockDim.x) {
+            const int slot = idx / (npi * 18), rem = idx - slot * (npi * 18), pc = rem / 18, nn = rem - pc * 18;
+            tc_b_values(P, Bbuf + (size_t)slot * bin_bytes, pc, tcls[pc], nn,
+                        Zs[(slot * npi + pc) * 9 + (nn >= 9 ? nn - 9 : nn)]);
         }
         tc::fence_async_smem();
         __syncthreads();
@@ -1634,6 +1625,13 @@ __global__ void __launch_bounds__(kThreads, 2) k4_work_tc(P4Params p) {
         const int* src = reinterpret_cast<const int*>(P);
         int* dst = reinterpret_cast<int*>(smem + TL.plan);
         for (int x = threadIdx.x; x < (int)(sizeof(TcPlan) / sizeof(int)); x += blockDim.x) dst[x] = src[x];
+        uint4* bz = reinterpret_cast<uint4*>(smem + TL.b);
+        for (int x = threadIdx.x; x < P->zbins * (P->bin_bytes >> 4); x += blockDim.x) bz[x] = make_uint4(0, 0, 0, 0);
+        int* tcls = reinterpret_cast<int*>(smem + TL.cls);
+        for (int pass = 0; pass < P->npass; pass++)
+            for (int b = P->pass_blk0[pass]; b < P->pass_blk0[pass + 1]; b++)
+                for (int pc = P->blk[b].x + threadIdx.x; pc < P->blk[b].y; pc += blockDim.x)
+                    tcls[pc] = pass << 16 | (b - P->pass_blk0[pass]);
     }
     if (threadIdx.x == 0) {
         tc::mbar_init(tc::smem_u32(&bars[0]), 1);
