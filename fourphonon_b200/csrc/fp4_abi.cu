@@ -194,9 +194,9 @@ static constexpr size_t kCopyMin = (size_t)8 << 20;  // below this the threads c
 
 int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
     size_t total = 0;
+    for (int x = 0; x < n; x++) total += list[x].bytes;
     bool pageable = true;
-    for (int x = 0; x < n; x++) {
-        total += list[x].bytes;
+    for (int x = 0; x < n && total >= kCopyMin; x++) {
         cudaPointerAttributes a{};
         if (list[x].bytes && cudaPointerGetAttributes(&a, list[x].host) == cudaSuccess)
             pageable = pageable && a.type == cudaMemoryTypeUnregistered;
@@ -460,7 +460,7 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
             std::stable_sort(kv.second.begin(), kv.second.end(), [&](int x, int y) { return atoms[x].y < atoms[y].y; });
         cls_grp[p] = (int)grp_start.size();
         for (int t : kv.second) {
-            if ((int)grp_start.size() == cls_grp[p] || grp_a2.back() != atoms[t].y) {
+            if (order == 4 && ((int)grp_start.size() == cls_grp[p] || grp_a2.back() != atoms[t].y)) {
                 grp_start.push_back((int)cl_index.size());
                 grp_a2.push_back(atoms[t].y);
             }
@@ -493,14 +493,17 @@ int fp4_setup_ifc(fp4_ctx* c, const fp4_globals* g, int order, int32_t ntri, con
         // phase tables exp(2 pi i x D_d / N_d), x in [0, N_d), of the axes where D_d is not a multiple of N_d
         std::vector<int4> cls_ph(npi);
         std::vector<int> pt_root;
+        std::map<int, int> table;  // (axis, D_d mod N_d) -> place: classes share their tables
         for (int q = 0; q < npi; q++) {
             const int D[3] = {pi_d[q].x, pi_d[q].y, pi_d[q].z};
             int place[3] = {0, 0, 0}, ntab = 0;
             for (int d = 0; d < 3; d++) {
                 const int N = g->ngrid[d], m = ((D[d] % N) + N) % N;
                 if (m == 0) continue;
-                place[ntab++] = (int)pt_root.size() | (8 * d) << 24;
-                for (int x = 0; x < N; x++) pt_root.push_back((d << 16) | (x * m % N));
+                const auto found = table.emplace((d << 16) | m, (int)pt_root.size());
+                if (found.second)
+                    for (int x = 0; x < N; x++) pt_root.push_back((d << 16) | (x * m % N));
+                place[ntab++] = found.first->second | (8 * d) << 24;
             }
             cls_ph[q] = make_int4(place[0], place[1], place[2], ntab);
         }
