@@ -113,17 +113,24 @@ def ref_flops_per_process(s):
     return 644.0 * s.ifc4.ntri + 40.0
 
 
-def executed_flops(s, counters, npi):
+def executed_flops(s, counters):
     """FP64 operations the main kernel executes, from its work counters: 27 per
-    broadening evaluation, 3 per window test, 27+25+12*nT+116*classes per
-    contracted process and nb*9*Ntri*98 per reciprocal cluster table build."""
+    broadening evaluation, 3 per window test; per contracted process 27+25+12*nT for
+    the weights and the contraction's complex multiply-adds (8 each): 9 per class, 3
+    more per class whose phase is not 1, 3 per third-phonon atom, and a product (6) per
+    further axis of a phase; per cluster table build of one branch, 20 per cluster entry
+    (27 of them) and 8 per term of each of its nb tables."""
     nproc, ncontr, nsig, ncand, nz = counters[:5]
-    nT = len(s.temperatures)
-    f_sigma = 27.0
-    f_test = 3.0
-    f_proc = 27.0 + 25.0 + 12.0 * nT + 116.0 * npi
-    f_z = s.nb * 9.0 * s.ifc4.ntri * 98.0  # per table build (one branch i, all j)
-    return nsig * f_sigma + ncand * f_test + ncontr * f_proc + nz * f_z
+    f = s.ifc4
+    classes, groups = {}, set()
+    for c in range(f.ntri):
+        key = (tuple(f.cells[1, c] - f.cells[2, c]), int(f.atoms[2, c]), int(f.atoms[3, c]))
+        classes[key] = sum(1 for d in range(3) if key[0][d] % s.ngrid[d] != 0)
+        groups.add(key + (int(f.atoms[1, c]),))
+    f_proc = 27.0 + 25.0 + 12.0 * len(s.temperatures) + 24.0 * len({k[1] for k in classes})
+    f_proc += sum(72.0 + (24.0 + 6.0 * (axes - 1) if axes else 0.0) for axes in classes.values())
+    f_z = 27.0 * 20.0 * f.ntri + 8.0 * 27.0 * len(groups) * s.nb
+    return nsig * 27.0 + ncand * 3.0 + ncontr * f_proc + nz * f_z
 
 
 def filter_stage(counters, kernel_ms, phase_a_frac, peak):
@@ -514,7 +521,7 @@ def run_ours(args):
     kms = float(np.mean([r["kms"] for r in res]))
     last = res[-1]
     cnt = last["counters"]
-    fl = executed_flops(s, cnt, npi)
+    fl = executed_flops(s, cnt)
     achieved = fl / (kms / 1e3) / 1e12
     launches = sum(r["launches"] for r in res)
 
