@@ -118,7 +118,7 @@ extern "C" int fp4_destroy(fp4_ctx* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     for (DevBuffer* b : c->all_buffers()) b->release();
-    if (c->staging) cudaFreeHost(c->staging);
+    fp4_close_lanes(c);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaEventDestroy(c->evk0);
@@ -184,55 +184,95 @@ extern "C" int fp4_set_upload_cache(fp4_ctx* c, int enable) {
 // ---------------------------------------------------------------------------
 // A process list is tens to hundreds of MB of pageable memory, and an output list is
 // often fresh, its pages not yet mapped.  A plain copy runs through the driver's staging
-// buffer on one thread, which also takes every page fault.  Here kCopyThreads threads
-// take chunks in turn, each with two pinned slots of its own, so that the transfers, the
-// host copies and the page faults of different chunks overlap: the three-phonon stage of
-// the 16^3 diamond grid, which moves 115 MB out and back in, takes 28 ms in place of 61.
+// buffer on one thread, which also takes every page fault.  Here up to kCopyThreads
+// threads take chunks in turn, each through a lane of its own (a stream and two pinned
+// slots), so that the transfers, the host copies and the page faults of different chunks
+// overlap.
+//   The lanes' streams wait for an event that the calling thread records on c->stream:
+// the caller's handle itself is used on the calling thread only, since cudaStreamPerThread
+// means another stream in each thread.
 static constexpr int kCopyThreads = 8;
 static constexpr size_t kCopyChunk = (size_t)1 << 20;
 static constexpr size_t kCopyMin = (size_t)8 << 20;  // below this the threads cost more than they save
 
+void fp4_close_lanes(fp4_ctx* c) {
+    for (auto& l : c->lanes) {
+        for (auto& v : l.done)
+            if (v) cudaEventDestroy(v);
+        if (l.stream) cudaStreamDestroy(l.stream);
+    }
+    c->lanes.clear();
+    if (c->ev_copy) cudaEventDestroy(c->ev_copy);
+    c->ev_copy = nullptr;
+    if (c->slots) cudaFreeHost(c->slots);
+    c->slots = nullptr;
+}
+
+static bool open_lanes(fp4_ctx* c, int n) {
+    cudaError_t e = cudaMallocHost(&c->slots, (size_t)n * 2 * kCopyChunk);
+    if (e != cudaSuccess) c->slots = nullptr;
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_copy, cudaEventDisableTiming);
+    c->lanes.resize(n);
+    for (int x = 0; x < n; x++) {
+        CopyLane& l = c->lanes[x];
+        l.slot = c->slots + (size_t)x * 2 * kCopyChunk;
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
+        for (auto& v : l.done)
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) return true;
+    fp4_close_lanes(c);
+    cudaGetLastError();
+    return false;
+}
+
+// Lanes for a copy of `total` bytes between the device and `list`; 0 or 1: a plain copy.
+static int copy_lanes(fp4_ctx* c, const HostCopy* list, int n, size_t total) {
+    if (total < kCopyMin) return 0;
+    for (int x = 0; x < n; x++) {
+        cudaPointerAttributes a{};
+        if (list[x].bytes && (cudaPointerGetAttributes(&a, list[x].host) != cudaSuccess ||
+                              a.type != cudaMemoryTypeUnregistered)) {
+            cudaGetLastError();
+            return 0;
+        }
+    }
+    const int want = std::min<int>(kCopyThreads, (int)std::thread::hardware_concurrency());
+    if (want < 2) return 0;
+    if (c->lanes.empty() && !open_lanes(c, want)) return 0;
+    return std::min(want, (int)c->lanes.size());
+}
+
 int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
     size_t total = 0;
     for (int x = 0; x < n; x++) total += list[x].bytes;
-    bool pageable = true;
-    for (int x = 0; x < n && total >= kCopyMin; x++) {
-        cudaPointerAttributes a{};
-        if (list[x].bytes && cudaPointerGetAttributes(&a, list[x].host) == cudaSuccess)
-            pageable = pageable && a.type == cudaMemoryTypeUnregistered;
-    }
-    const int nthr = std::min<int>(kCopyThreads, (int)std::thread::hardware_concurrency());
-    if (pageable && total >= kCopyMin && nthr > 1 && !c->staging &&
-        cudaMallocHost(&c->staging, 2 * kCopyThreads * kCopyChunk) != cudaSuccess) {
-        c->staging = nullptr;
-        cudaGetLastError();
-    }
-    if (!pageable || total < kCopyMin || nthr <= 1 || !c->staging) {
+    const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+    const int nthr = copy_lanes(c, list, n, total);
+    if (nthr < 2) {
         for (int x = 0; x < n; x++)
             if (list[x].bytes)
                 CK(cudaMemcpyAsync(to_host ? list[x].host : list[x].dev, to_host ? list[x].dev : list[x].host,
-                                   list[x].bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, c->stream));
+                                   list[x].bytes, kind, c->stream));
         return FP4_OK;
     }
+    CK(cudaEventRecord(c->ev_copy, c->stream));
     std::vector<size_t> first(n + 1, 0);  // chunks before each copy
     for (int x = 0; x < n; x++) first[x + 1] = first[x] + (list[x].bytes + kCopyChunk - 1) / kCopyChunk;
     std::atomic<size_t> next{0};
     std::atomic<int> failed{(int)cudaSuccess};
     auto work = [&](int id) {
+        const CopyLane& lane = c->lanes[id];
         cudaError_t e = cudaSetDevice(c->device);
-        cudaEvent_t ev[2] = {nullptr, nullptr};
-        for (auto& v : ev)
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
-        unsigned char* slot[2] = {c->staging + (size_t)(2 * id) * kCopyChunk,
-                                  c->staging + (size_t)(2 * id + 1) * kCopyChunk};
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(lane.stream, c->ev_copy, 0);
         struct Pending {
             void* host;
             size_t bytes;
         } pend[2] = {{nullptr, 0}, {nullptr, 0}};
+        auto slot = [&](int s) { return lane.slot + (size_t)s * kCopyChunk; };
         auto finish = [&](int s) {  // the transfer of slot s is over; to the host: hand its bytes on
             if (e == cudaSuccess && pend[s].bytes) {
-                e = cudaEventSynchronize(ev[s]);
-                if (e == cudaSuccess && to_host) memcpy(pend[s].host, slot[s], pend[s].bytes);
+                e = cudaEventSynchronize(lane.done[s]);
+                if (e == cudaSuccess && to_host) memcpy(pend[s].host, slot(s), pend[s].bytes);
             }
             pend[s].bytes = 0;
         };
@@ -246,17 +286,17 @@ int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
             unsigned char* d = static_cast<unsigned char*>(list[x].dev) + off;
             finish(s);
             if (e != cudaSuccess) break;
-            if (!to_host) memcpy(slot[s], h, m);
-            e = cudaMemcpyAsync(to_host ? slot[s] : d, to_host ? d : slot[s], m,
-                                to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, c->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(ev[s], c->stream);
+            if (!to_host) memcpy(slot(s), h, m);
+            e = cudaMemcpyAsync(to_host ? slot(s) : d, to_host ? d : slot(s), m, kind, lane.stream);
+            if (e == cudaSuccess) e = cudaEventRecord(lane.done[s], lane.stream);
             pend[s] = {h, m};
         }
         finish(0);
         finish(1);
-        for (auto& v : ev)
-            if (v) cudaEventDestroy(v);
-        if (e != cudaSuccess) failed = (int)e;
+        if (e != cudaSuccess) {  // nothing of this lane stays in flight behind an error
+            failed = (int)e;
+            cudaStreamSynchronize(lane.stream);
+        }
     };
     std::vector<std::thread> pool;
     try {

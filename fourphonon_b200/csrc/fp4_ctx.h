@@ -50,6 +50,13 @@ struct IfcTables {
     }
 };
 
+// One host thread's way between pageable and device memory.
+struct CopyLane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done[2] = {nullptr, nullptr};  // the last transfer of each slot
+    unsigned char* slot = nullptr;             // two pinned slots
+};
+
 struct fp4_ctx {
     int device = 0;
     int sm_count = 148;
@@ -69,7 +76,9 @@ struct fp4_ctx {
     DevBuffer b_energy, b_velocity, b_wv, b_eigraw, b_eig, b_eigf, b_list, b_qc, b_root[3], b_rootf[3];
     DevBuffer b_temps, b_bose, b_wb, b_out, b_out4, b_lists, b_gamma, b_off, b_counts;
     DevBuffer b_queue, b_part, b_work, b_err, b_stats;
-    unsigned char* staging = nullptr;  // pinned staging of fp4_copy_lists
+    std::vector<CopyLane> lanes;       // of fp4_copy_lists, opened by the first large list
+    unsigned char* slots = nullptr;    // their pinned memory
+    cudaEvent_t ev_copy = nullptr;     // what c->stream held when the lanes' copies began
     DevBuffer b_tcplan, b_wtab;  // tensor-core contraction: its plan and phase rows
     bool last_tc = false;        // the last four-phonon RTA call ran its contraction on the tensor cores
     DevBuffer b_bte[13];  // [12]: the new iterate of a Jacobi sweep
@@ -102,9 +111,11 @@ struct HostCopy {
     void* dev;
     size_t bytes;
 };
-// Copies in stream order, all to the host or all to the device.  Large ones go through the
-// context's pinned buffer with several host threads; they are done when the call returns.
+// Copies all to the host or all to the device, after everything that c->stream holds.
+// Large ones go through the context's lanes with several host threads and are done when the
+// call returns; others are queued on c->stream.
 int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host);
+void fp4_close_lanes(fp4_ctx* c);
 
 int fp4_fail(fp4_ctx* c, int code, const char* fmt, ...);
 int fp4_begin(fp4_ctx* c);
