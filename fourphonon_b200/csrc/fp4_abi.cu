@@ -7,6 +7,7 @@
 // results back into the caller's arrays.  Failures return a negative code
 // and leave a message for fp4_last_error(); nothing falls back to the CPU.
 #include <cuda_runtime.h>
+#include <sched.h>
 
 #include <algorithm>
 #include <atomic>
@@ -191,9 +192,23 @@ extern "C" int fp4_set_upload_cache(fp4_ctx* c, int enable) {
 //   The lanes' streams wait for an event that the calling thread records on c->stream:
 // the caller's handle itself is used on the calling thread only, since cudaStreamPerThread
 // means another stream in each thread.
+//   When (16 usable processors; ms of Ind_driver, whose lists go to the host, into pages
+// that are fresh or already mapped, and of a Jacobi sweep, whose lists go to the device;
+// plain copies, then lanes that are open; fresh: a first call less 12 ms for the pinning):
+//               fresh        mapped       to the device
+//     8.5 MB    6.5,  -       2.7,  2.8    1.0, 0.9
+//      31 MB   14.8,  8       7.7,  6.9    3.0, 2.3
+//     110 MB   41,   19      21.4, 19.3   14.4, 7.6
+// so below kCopyMin the threads save nothing.  Pinning the slots takes 9 to 17 ms, which
+// the lanes save again over about 80 MB to fresh pages or 250 MB to the device: they are
+// opened when a context has copied kCopyOpen bytes of such lists, one to the host counted
+// three times, so that a context that copies a short list or two does not pay for them
+// (first call, 110 MB to fresh pages: 41 ms plain, 26 to 31 with the pinning; 31 MB: 15, 21).
+// Slots of 512 KB would take half as long to pin, and a 110 MB sweep 1.1 ms longer.
 static constexpr int kCopyThreads = 8;
 static constexpr size_t kCopyChunk = (size_t)1 << 20;
-static constexpr size_t kCopyMin = (size_t)8 << 20;  // below this the threads cost more than they save
+static constexpr size_t kCopyMin = (size_t)16 << 20;
+static constexpr size_t kCopyOpen = (size_t)256 << 20;
 
 void fp4_close_lanes(fp4_ctx* c) {
     for (auto& l : c->lanes) {
@@ -226,8 +241,15 @@ static bool open_lanes(fp4_ctx* c, int n) {
     return false;
 }
 
+// Processors that this process may run on (its affinity mask, which an MPI launcher sets).
+static int usable_cpus() {
+    cpu_set_t set;
+    if (sched_getaffinity(0, sizeof set, &set) == 0) return CPU_COUNT(&set);
+    return (int)std::thread::hardware_concurrency();
+}
+
 // Lanes for a copy of `total` bytes between the device and `list`; 0 or 1: a plain copy.
-static int copy_lanes(fp4_ctx* c, const HostCopy* list, int n, size_t total) {
+static int copy_lanes(fp4_ctx* c, const HostCopy* list, int n, size_t total, bool to_host) {
     if (total < kCopyMin) return 0;
     for (int x = 0; x < n; x++) {
         cudaPointerAttributes a{};
@@ -237,9 +259,13 @@ static int copy_lanes(fp4_ctx* c, const HostCopy* list, int n, size_t total) {
             return 0;
         }
     }
-    const int want = std::min<int>(kCopyThreads, (int)std::thread::hardware_concurrency());
+    const int want = std::min(kCopyThreads, usable_cpus());
     if (want < 2) return 0;
-    if (c->lanes.empty() && !open_lanes(c, want)) return 0;
+    c->list_bytes += to_host ? 3 * total : total;
+    if (c->lanes.empty() && (c->list_bytes < kCopyOpen || !open_lanes(c, want))) {
+        if (c->list_bytes >= kCopyOpen) c->list_bytes = 0;  // no memory for them: not again for a while
+        return 0;
+    }
     return std::min(want, (int)c->lanes.size());
 }
 
@@ -247,7 +273,7 @@ int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
     size_t total = 0;
     for (int x = 0; x < n; x++) total += list[x].bytes;
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
-    const int nthr = copy_lanes(c, list, n, total);
+    const int nthr = copy_lanes(c, list, n, total, to_host);
     if (nthr < 2) {
         for (int x = 0; x < n; x++)
             if (list[x].bytes)

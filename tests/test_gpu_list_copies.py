@@ -4,6 +4,7 @@ on every kind of stream, against the same calls on short lists, which are copied
 The 16^3 diamond lists hold 110 MB, so that each thread uses each of its pinned slots
 many times over, also where the threads wait for a context to have copied 256 MB."""
 import dataclasses
+import os
 
 import numpy as np
 import pytest
@@ -77,4 +78,20 @@ def test_lists_to_the_device(solve, handle):
         scale = np.abs(want).max()
         assert np.abs(half - (want - 0.5 * zero)).max() <= 1e-13 * scale
     finally:
+        c.close()
+
+
+def test_one_usable_processor(solve):
+    """A process bound to one processor copies plainly, and to the same lists."""
+    s, n_p, n_m, want = solve
+    mask = os.sched_getaffinity(0)
+    c = abi.Context(0)
+    try:
+        os.sched_setaffinity(0, {min(mask)})
+        for _ in range(3):
+            got = c.ind_driver(s, n_p, n_m)
+        for k in LISTS:
+            assert np.array_equal(got[k], want[k]), k
+    finally:
+        os.sched_setaffinity(0, mask)
         c.close()
