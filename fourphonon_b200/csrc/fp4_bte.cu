@@ -631,7 +631,8 @@ static size_t block_smem(int nb, int pts) { return (size_t)pts * (nb * 3 + 9) * 
 // Cuts the irreducible points into blocks of at most kBlockPoints points (or one star),
 // and lays out their steps and, for the worst case that every term falls inside the
 // block, their listed terms; terms, steps and pts are the largest block's.  False when a
-// block's terms or points would take too much memory: the sweep then runs on k_sweep.
+// block's terms or points would take too much memory, or when there are more branches than
+// k_block_steps has threads: the sweep then runs on k_sweep.
 static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* n_plus, const int32_t* n_minus,
                         std::vector<int>& cut, std::vector<int>& step0, std::vector<long long>& term0, size_t& terms,
                         size_t& steps, int& pts) {
@@ -663,7 +664,7 @@ static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* 
         pts = std::max(pts, bp);
     }
     cut.push_back(nlist);
-    return terms <= kMaxTerms && block_smem(nb, pts) <= kMaxSmem;
+    return nb <= kStepThreads && terms <= kMaxTerms && block_smem(nb, pts) <= kMaxSmem;
 }
 
 static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int32_t* nequi, const int32_t* allequi,

@@ -1,0 +1,64 @@
+"""The in-order three-phonon sweep on process lists that are made up, against the oracle's
+sequential sweep: what Ind_driver's lists of small cells do not reach."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import helpers as H
+import oracle as O
+from fourphonon_b200 import abi
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+def _solve(grid, natoms):
+    """The wedge and symmetrizers of the diamond grid with 3 natoms branches of random
+    frequencies and velocities."""
+    s = H.cached_solve("diamond", grid)
+    rng = np.random.default_rng(natoms)
+    nb = 3 * natoms
+    cr = dataclasses.replace(s.crystal, positions=np.zeros((3, natoms)), types=np.ones(natoms, dtype=np.int64),
+                             masses=np.ones(1))
+    return dataclasses.replace(s, crystal=cr, energy=np.asfortranarray(rng.uniform(1.0, 10.0, (s.nptk, nb))),
+                               velocity=np.asfortranarray(rng.normal(size=(s.nptk, nb, 3))),
+                               eig=np.zeros((s.nptk, nb, 1), dtype=np.complex128), ifc3=None, ifc4=None)
+
+
+def _lists(s, n_plus, n_minus, seed):
+    """Random processes, n_plus and n_minus of each mode; each mode's amplitudes sum to at
+    most a quarter, so that a sweep of tau = 1 halves a difference at least."""
+    rng = np.random.default_rng(seed)
+    d = {}
+    for k, n in (("plus", n_plus), ("minus", n_minus)):
+        t = int(n.sum())
+        d["ind2_" + k] = rng.integers(1, s.nptk * s.nb + 1, t, dtype=np.int32)
+        d["ind3_" + k] = rng.integers(1, s.nptk * s.nb + 1, t, dtype=np.int32)
+        d["gamma_" + k] = rng.uniform(0.0, 0.125, t) / np.repeat(np.maximum(n, 1), n)
+    return d
+
+
+def _compare(s, n_plus, n_minus, seed=1):
+    lists = _lists(s, n_plus, n_minus, seed)
+    tau = np.random.default_rng(seed + 1).uniform(0.5, 1.0, s.nmodes)
+    ctx = abi.Context(0)
+    try:
+        F0 = ctx.iteration0(s, tau)
+        got = ctx.iteration(s, F0.copy(), tau, n_plus, n_minus, lists)
+    finally:
+        ctx.close()
+    want = O.Oracle(s).iteration(F0.copy(), tau, n_plus, n_minus, lists)
+    # a sum of n terms in another order: n eps of the terms' magnitudes, whose sum is at
+    # most the largest |F|; the sweep at most doubles what a step brings in
+    rtol = 2.0 * EPS * 2 * int(max(n_plus.max(), n_minus.max()) + 64)
+    assert np.abs(got - want).max() <= rtol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("natoms", [42, 43, 86])
+def test_many_branches(natoms):
+    """126, 129 and 258 branches: fewer and more than the threads of the sweep's chain."""
+    s = _solve((2, 2, 2), natoms)
+    n = np.random.default_rng(natoms).integers(0, 40, (2, s.nmodes)).astype(np.int32)
+    _compare(s, n[0], n[1])
