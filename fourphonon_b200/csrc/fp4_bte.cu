@@ -240,10 +240,13 @@ __global__ void k_block_begin(BteParams p, BlockParams q, int l1) {
     mark_block(p, q, 0, l1);
 }
 
-// One CTA per step of the block [l0, l1).
-__global__ void __launch_bounds__(256) k_block_sums(BteParams p, BlockParams q, int l0, int l1) {
+// One CTA per step of the block [l0, l1).  The listed terms keep a fixed order (by rows of
+// kSumThreads processes, warp and lane, each warp's first terms before its second ones), so
+// that a sweep gives the same bits every time.
+constexpr int kSumThreads = 256;
+__global__ void __launch_bounds__(kSumThreads) k_block_sums(BteParams p, BlockParams q, int l0, int l1) {
     __shared__ double red[3][32];
-    __shared__ int s_cnt;
+    __shared__ int s_cnt[2][kSumThreads / 32];  // each warp's listed terms of a row, alternately
     const int nb = p.nb;
     const int step = q.step0[l0] + blockIdx.x;
     int ll = l0;
@@ -255,37 +258,66 @@ __global__ void __launch_bounds__(256) k_block_sums(BteParams p, BlockParams q, 
     const long long op = p.off_plus[mm], om = p.off_minus[mm];
     const long long out = q.term0[mm] + (long long)kk * 2 * nt;
     const int lim = p.nptk * nb;
-    if (threadIdx.x == 0) s_cnt = 0;
-    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
     double a[3] = {0.0, 0.0, 0.0};
     const size_t pl = (size_t)lim;
-    auto term = [&](int b, int qx, double g) {  // g F(b, qx), or its entry in the list
-        const int slot = q.slot_of[qx];
-        if (slot >= 0) {
-            const int pos = atomicAdd(&s_cnt, 1);  // at most 2 nt terms
-            q.idx[out + pos] = slot * nb + b;
-            q.coef[out + pos] = g;
-        } else {
-            const double* f = p.F + (size_t)qx * nb + b;
-            a[0] = fma(g, f[0], a[0]);
-            a[1] = fma(g, f[pl], a[1]);
-            a[2] = fma(g, f[2 * pl], a[2]);
+    int listed = 0;
+    for (int x0 = 0, buf = 0; x0 < nt; x0 += kSumThreads, buf ^= 1) {
+        const int x = x0 + threadIdx.x;
+        int ia = -1, ib = -1;  // the process's listed terms: slot * nb + branch
+        double g = 0.0, gb = 0.0;
+        if (x < nt) {
+            const bool plus = x < np_;
+            const long long o = plus ? op + x : om + (x - np_);
+            const int x2 = (plus ? p.i2p : p.i2m)[o] - 1, x3 = (plus ? p.i3p : p.i3m)[o] - 1;
+            if (x2 < 0 || x2 >= lim || x3 < 0 || x3 >= lim) {
+                atomicOr(p.err, kErrList);
+            } else {
+                const int m2 = x2 / nb, j = x2 - m2 * nb, n3 = x3 / nb, k = x3 - n3 * nb;
+                const int qa = p.id_equi[(size_t)n3 * p.nsr + sym] - 1, qb = p.id_equi[(size_t)m2 * p.nsr + sym] - 1;
+                const int sa = q.slot_of[qa], sb = q.slot_of[qb];
+                const double* fa = p.F + (size_t)qa * nb + k;
+                const double* fb = p.F + (size_t)qb * nb + j;
+                g = plus ? p.gp[o] : p.gm[o] * 5.e-1;
+                gb = plus ? -g : g;
+                if (sa < 0 && sb < 0) {  // as step_sum: the amplitude times F_a -+ F_b
+                    const double sg = plus ? -1.0 : 1.0;
+#pragma unroll
+                    for (int d = 0; d < 3; d++) a[d] = fma(g, fma(sg, fb[d * pl], fa[d * pl]), a[d]);
+                } else {
+                    if (sa >= 0)
+                        ia = sa * nb + k;
+                    else
+                        for (int d = 0; d < 3; d++) a[d] = fma(g, fa[d * pl], a[d]);
+                    if (sb >= 0)
+                        ib = sb * nb + j;
+                    else
+                        for (int d = 0; d < 3; d++) a[d] = fma(gb, fb[d * pl], a[d]);
+                }
+            }
         }
-    };
-    for (int x = threadIdx.x; x < nt; x += blockDim.x) {
-        const bool plus = x < np_;
-        const long long o = plus ? op + x : om + (x - np_);
-        const int x2 = (plus ? p.i2p : p.i2m)[o] - 1, x3 = (plus ? p.i3p : p.i3m)[o] - 1;
-        if (x2 < 0 || x2 >= lim || x3 < 0 || x3 >= lim) {
-            atomicOr(p.err, kErrList);
-            continue;
+        const unsigned ma = __ballot_sync(0xffffffffu, ia >= 0), mb = __ballot_sync(0xffffffffu, ib >= 0);
+        if (lane == 0) s_cnt[buf][warp] = __popc(ma) + __popc(mb);
+        __syncthreads();  // (the next row writes the other counts)
+        int pos = listed;
+#pragma unroll
+        for (int w = 0; w < kSumThreads / 32; w++) {
+            const int n = s_cnt[buf][w];
+            pos += w < warp ? n : 0;
+            listed += n;
         }
-        const int m2 = x2 / nb, n3 = x3 / nb;
-        const double g = plus ? p.gp[o] : p.gm[o] * 5.e-1;
-        term(x3 - n3 * nb, p.id_equi[(size_t)n3 * p.nsr + sym] - 1, g);
-        term(x2 - m2 * nb, p.id_equi[(size_t)m2 * p.nsr + sym] - 1, plus ? -g : g);
+        if (ia >= 0) {
+            q.idx[out + pos + __popc(ma & below)] = ia;
+            q.coef[out + pos + __popc(ma & below)] = g;
+        }
+        pos += __popc(ma);
+        if (ib >= 0) {
+            q.idx[out + pos + __popc(mb & below)] = ib;
+            q.coef[out + pos + __popc(mb & below)] = gb;
+        }
     }
-    block_sum3(a[0], a[1], a[2], red);  // its barrier also ends the appends
+    block_sum3(a[0], a[1], a[2], red);
     if (threadIdx.x == 0) {
         const double tz = p.tau_zero[mm];
         const size_t e = (size_t)i * p.nptk + qq;
@@ -297,7 +329,7 @@ __global__ void __launch_bounds__(256) k_block_sums(BteParams p, BlockParams q, 
         }
         s.tau = tz;
         s.term = out;
-        s.cnt = s_cnt;
+        s.cnt = listed;
         s.slot = q.slot_of[qq];
         s.band = i;
         q.info[blockIdx.x] = s;
@@ -852,7 +884,7 @@ static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int3
             const int l0 = cut[x], l1 = cut[x + 1], l2 = x + 2 < cut.size() ? cut[x + 2] : l1;
             const int ns = step0[l1] - step0[l0];
             if (ns) {
-                k_block_sums<<<ns, 256, 0, c->stream>>>(p, q, l0, l1);
+                k_block_sums<<<ns, kSumThreads, 0, c->stream>>>(p, q, l0, l1);
                 CK(cudaGetLastError());
                 c->launches++;
             }

@@ -62,3 +62,20 @@ def test_many_branches(natoms):
     s = _solve((2, 2, 2), natoms)
     n = np.random.default_rng(natoms).integers(0, 40, (2, s.nmodes)).astype(np.int32)
     _compare(s, n[0], n[1])
+
+
+def test_the_same_bits_every_time():
+    """The terms inside a block are listed, and summed, in a fixed order."""
+    s = _solve((6, 6, 6), 2)
+    n = np.random.default_rng(3).integers(300, 900, (2, s.nmodes)).astype(np.int32)
+    lists = _lists(s, n[0], n[1], 5)
+    tau = np.random.default_rng(4).uniform(0.5, 1.0, s.nmodes)
+    ctx = abi.Context(0)
+    try:
+        F0 = ctx.iteration0(s, tau)
+        first = ctx.iteration(s, F0.copy(), tau, n[0], n[1], lists)
+        for _ in range(8):
+            assert np.array_equal(ctx.iteration(s, F0.copy(), tau, n[0], n[1], lists), first)
+    finally:
+        ctx.close()
+    _compare(s, n[0], n[1])
