@@ -664,7 +664,9 @@ static size_t block_smem(int nb, int pts) { return (size_t)pts * (nb * 3 + 9) * 
 // and lays out their steps and, for the worst case that every term falls inside the
 // block, their listed terms; terms, steps and pts are the largest block's.  False when a
 // block's terms or points would take too much memory, or when there are more branches than
-// k_block_steps has threads: the sweep then runs on k_sweep.
+// k_block_steps has threads: the sweep then runs on k_sweep.  (The worst case is far from
+// the listed share of about B / nptk: the 12^3 diamond grid gets 20 MB and lists 4 % of it.
+// One star of 48 points passes the limit when its modes have 350,000 processes in all.)
 static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* n_plus, const int32_t* n_minus,
                         std::vector<int>& cut, std::vector<int>& step0, std::vector<long long>& term0, size_t& terms,
                         size_t& steps, int& pts) {
@@ -856,14 +858,18 @@ static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int3
     std::vector<long long> term0;
     size_t terms = 0, steps = 0;
     int pts = 0;
-    const bool blocks = !l4 && plan_blocks(nb, nlist, nequi, n_plus, n_minus, cut, step0, term0, terms, steps, pts);
+    bool blocks = !l4 && plan_blocks(nb, nlist, nequi, n_plus, n_minus, cut, step0, term0, terms, steps, pts);
+    // [slot_of | step0] and [term0], [records], [coef], [idx] in one buffer
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t o1 = up((size_t)nptk * sizeof(int)), o2 = o1 + up((nlist + 1) * sizeof(int)),
+                 o3 = o2 + up(nm * sizeof(long long)), o4 = o3 + up(steps * sizeof(StepInfo)),
+                 o5 = o4 + up(terms * sizeof(double)), o6 = o5 + up(terms * sizeof(int));
+    if (blocks && B[12].reserve(c, o6) != FP4_OK) {  // no room: k_sweep needs none
+        cudaGetLastError();
+        c->err.clear();
+        blocks = false;
+    }
     if (blocks) {
-        // [slot_of | step0] and [term0], [records], [idx], [coef] in one buffer
-        auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-        const size_t o1 = up((size_t)nptk * sizeof(int)), o2 = o1 + up((nlist + 1) * sizeof(int)),
-                     o3 = o2 + up(nm * sizeof(long long)), o4 = o3 + up(steps * sizeof(StepInfo)),
-                     o5 = o4 + up(terms * sizeof(double)), o6 = o5 + up(terms * sizeof(int));
-        if ((r = B[12].reserve(c, o6))) return r;
         unsigned char* d = B[12].as<unsigned char>();
         BlockParams q{};
         q.slot_of = reinterpret_cast<int*>(d);

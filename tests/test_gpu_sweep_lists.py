@@ -79,3 +79,40 @@ def test_the_same_bits_every_time():
     finally:
         ctx.close()
     _compare(s, n[0], n[1])
+
+
+def _one_heavy_star(count):
+    """The 6^3 diamond solve, with count absorption and count emission processes in each mode of its
+    largest star (24 points) and 20 elsewhere."""
+    s = _solve((6, 6, 6), 2)
+    n = np.full((s.nlist, s.nb), 20, dtype=np.int32)
+    ll = int(np.argmax(s.wedge.nequi))
+    assert s.wedge.nequi[ll] == 24
+    n[ll] = count
+    return s, n.ravel()
+
+
+@pytest.mark.parametrize("count", [58_000, 59_000])
+def test_the_limit_of_the_listed_terms(count):
+    """Just below and just above 32 Mi terms of one star, from where the sequential kernel runs."""
+    assert (2 * 2 * 58_000 * 6 * 24 < 32 << 20) and (2 * 2 * 59_000 * 6 * 24 > 32 << 20)
+    s, n = _one_heavy_star(count)
+    _compare(s, n, n.copy())
+
+
+def test_no_memory_for_the_listed_terms():
+    """A sweep that finds no room for its terms (276 MB here) runs on the sequential kernel."""
+    import torch
+
+    s, n = _one_heavy_star(40_000)
+    _compare(s, n, n.copy())  # with room; loads the kernels
+    small = _solve((2, 2, 2), 43)
+    _compare(small, np.zeros(small.nmodes, np.int32), np.zeros(small.nmodes, np.int32))
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - (160 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 200 << 20
+        _compare(s, n, n.copy())
+    finally:
+        del hog
+        torch.cuda.empty_cache()
