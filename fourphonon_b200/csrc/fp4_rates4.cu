@@ -650,6 +650,14 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
             }
             const double* r1 = p.wb + (size_t)(ii * nb + j) * wb_stride(NT);
             my_contr += own;
+            double wl = 0.0;  // LIST, one temperature: WP4, formed once
+            if constexpr (LIST) {
+                if (own) {
+                    wl = k4_wp4(g, r1, ch, 0);
+                    p.gamma_out[ch][qpos[qi]] = wl * v2 * p.gamma_scale;
+                }
+            }
+            auto wp4_of = [&](int t) { return LIST ? wl : k4_wp4(g, r1, ch, t); };
             // the warp's branch, or branches i_lo..i_hi where the warp meets a boundary
             if (!__all_sync(0xffffffffu, i == cur_i)) {
                 const int i_lo = __shfl_sync(0xffffffffu, i, 0), i_hi = __shfl_sync(0xffffffffu, i, 31);
@@ -666,8 +674,7 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
 #pragma unroll
                     for (int t = 0; t < NT; t++)
                         if (NT <= 2 || t < nT) {
-                            const double wp4 = own ? k4_wp4(g, r1, ch, t) : 0.0;
-                            if (LIST && own) p.gamma_out[ch][qpos[qi]] = wp4 * v2 * p.gamma_scale;
+                            const double wp4 = own ? wp4_of(t) : 0.0;
                             for (int x = i_lo; x <= i_hi; x++)
                                 add_warp(x, t, (own && i == x) ? wp4 * v2 : 0.0, (own && i == x) ? wp4 : 0.0);
                         }
@@ -678,8 +685,7 @@ __device__ __noinline__ int k4_phase_b(const unsigned long long* qbase, const do
 #pragma unroll
                 for (int t = 0; t < NT; t++)
                     if (NT <= 2 || t < nT) {
-                        const double wp4 = k4_wp4(g, r1, ch, t);
-                        if (LIST) p.gamma_out[ch][qpos[qi]] = wp4 * v2 * p.gamma_scale;
+                        const double wp4 = wp4_of(t);
                         accr[t] = fma(wp4, v2, accr[t]);
                         accw[t] += wp4;
                     }
@@ -1097,53 +1103,63 @@ __device__ void k4_list_segment(const P4Params& p, unsigned char* smem, const La
     __syncthreads();
     const long long total = segpre[nb];
     const long long lim = (long long)nptk * nb;
-    int iter = 0;
-    for (long long base = 0; base < total; base += blockDim.x, iter++) {
-        if ((iter % kCheckEvery) == 0 && queue_nearly_full(p, cnt, nb2, misc))
-            k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
-        const long long e = base + threadIdx.x;
-        if (e >= total) continue;
-        int i = 0;
-        while (i + 1 < nb && segpre[i + 1] <= e) i++;
-        const long long pos = seglo[i] + (e - segpre[i]);
-        const long long x2 = I2[pos] - 1, x3 = I3[pos] - 1, x4 = I4[pos] - 1;
-        bool ok = x2 >= 0 && x2 < lim && x3 >= 0 && x3 < lim && x4 >= 0 && x4 < lim && x2 / nb == ii;
-        const int j = (int)(x2 % nb), jj = (int)(x3 / nb), k = (int)(x3 % nb), ss = (int)(x4 / nb), l = (int)(x4 % nb);
-        int a = 0, b = 0, c = 0;
-        if (ok) {
-            q_coords_t(S, jj, a, b, c);
-            int t0, t1, t2;
-            if (ch == 0) {
-                t0 = n0 + m0 + a; t1 = n1 + m1 + b; t2 = n2 + m2 + c;
-            } else if (ch == 1) {
-                t0 = n0 + m0 - a; t1 = n1 + m1 - b; t2 = n2 + m2 - c;
-            } else {
-                t0 = n0 - m0 - a; t1 = n1 - m1 - b; t2 = n2 - m2 - c;
+    // Segments, as in phase A of the other kernels: entries until a queue is nearly full or
+    // the list ends, then phase B.  With the call inside the loop its state was spilled
+    // around it (Ind_driver_4ph in mixed precision, diamond 6^3: 5.81 ms, 5.63 so; a random
+    // 4-atom cell on 3^3: 2.29, 2.21).
+    for (long long seg = 0; seg < total;) {
+        long long base = seg;
+        seg = total;
+        for (int iter = 0; base < total; base += blockDim.x, iter++) {
+            if (iter > 0 && (iter % kCheckEvery) == 0 && queue_nearly_full(p, cnt, nb2, misc)) {
+                seg = base;
+                break;
             }
-            ok = q_index(S, wrapN(t0, N0), wrapN(t1, N1), wrapN(t2, N2)) == ss;
+            const long long e = base + threadIdx.x;
+            if (e >= total) continue;
+            int i = 0;
+            while (i + 1 < nb && segpre[i + 1] <= e) i++;
+            const long long pos = seglo[i] + (e - segpre[i]);
+            const long long x2 = I2[pos] - 1, x3 = I3[pos] - 1, x4 = I4[pos] - 1;
+            bool ok = x2 >= 0 && x2 < lim && x3 >= 0 && x3 < lim && x4 >= 0 && x4 < lim && x2 / nb == ii;
+            const int j = (int)(x2 % nb), jj = (int)(x3 / nb), k = (int)(x3 % nb);
+            const int ss = (int)(x4 / nb), l = (int)(x4 % nb);
+            int a = 0, b = 0, c = 0;
+            if (ok) {
+                q_coords_t(S, jj, a, b, c);
+                int t0, t1, t2;
+                if (ch == 0) {
+                    t0 = n0 + m0 + a; t1 = n1 + m1 + b; t2 = n2 + m2 + c;
+                } else if (ch == 1) {
+                    t0 = n0 + m0 - a; t1 = n1 + m1 - b; t2 = n2 + m2 - c;
+                } else {
+                    t0 = n0 - m0 - a; t1 = n1 - m1 - b; t2 = n2 - m2 - c;
+                }
+                ok = q_index(S, wrapN(t0, N0), wrapN(t1, N1), wrapN(t2, N2)) == ss;
+            }
+            if (!ok) {
+                atomicOr(p.err, kErrList);
+                continue;
+            }
+            my_surv++;
+            const double w1 = S.wv[ii * nb + j].w;
+            const double4 w2 = S.wv[jj * nb + k];
+            const double4 w3 = S.wv[ss * nb + l];
+            if (w1 <= 1.25 || w2.w <= 1.25 || w3.w <= 1.25) continue;  // WP4 = 0, Gamma = 0 (output pre-zeroed)
+            const int idx = i * nb + j;
+            const int qp = atomicAdd(&cnt[idx], 1);
+            if (qp >= p.subcap) {  // cannot happen with the capacity checks; never write past the bin
+                atomicOr(p.err, kErrQueue);
+                continue;
+            }
+            const size_t qi = (size_t)idx * p.subcap + qp;
+            qbase[qi] = pack_proc(a, b, c, ss, k, l);
+            qsig[qi] = sigma_exact(S, w2, w3);
+            qpos[qi] = pos;
         }
-        if (!ok) {
-            atomicOr(p.err, kErrList);
-            continue;
-        }
-        my_surv++;
-        const double w1 = S.wv[ii * nb + j].w;
-        const double4 w2 = S.wv[jj * nb + k];
-        const double4 w3 = S.wv[ss * nb + l];
-        if (w1 <= 1.25 || w2.w <= 1.25 || w3.w <= 1.25) continue;  // WP4 = 0, Gamma = 0 (output pre-zeroed)
-        const int idx = i * nb + j;
-        const int qp = atomicAdd(&cnt[idx], 1);
-        if (qp >= p.subcap) {  // cannot happen with the capacity checks; never write past the bin
-            atomicOr(p.err, kErrQueue);
-            continue;
-        }
-        const size_t qi = (size_t)idx * p.subcap + qp;
-        qbase[qi] = pack_proc(a, b, c, ss, k, l);
-        qsig[qi] = sigma_exact(S, w2, w3);
-        qpos[qi] = pos;
+        __syncthreads();
+        k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
     }
-    __syncthreads();
-    k4_flush<NT, MIXED, true, false>(p, smem, L, qbase, qsig, qpos, ch, ii, q0, my_contr);
 }
 
 // Per-thread work counters of one kernel, flushed into a P4Params::stats array.
