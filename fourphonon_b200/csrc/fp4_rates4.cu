@@ -109,12 +109,23 @@ constexpr int kStageSlots = 32;
 // Cells of the lookup table over the range of the sorted pair sums (phase A): with 36
 // sums of 2-atom cells a window then holds 0.1 to 0.2 sums that the exact test drops.
 constexpr int kCells = 256;
-__host__ __device__ inline int stage_passes(int nb2) {
+__host__ __device__ constexpr int stage_passes(int nb2) {
     int P = 8;
     while (P > 1 && (P * 256 - 1) / nb2 + 2 > kStageSlots) P >>= 1;
     return P;
 }
-__host__ __device__ inline int stage_slots(int nb2) { return (stage_passes(nb2) * 256 - 1) / nb2 + 2; }
+__host__ __device__ constexpr int stage_slots(int nb2) { return (stage_passes(nb2) * 256 - 1) / nb2 + 2; }
+__host__ __device__ constexpr size_t stage_bytes(int nb) { return (size_t)stage_slots(nb * nb) * 2 * nb * 32; }
+
+// Cluster groups (27 complex values each) that fit in the stage when phase B builds its
+// tables there: 13 at 3 branches, 16 to 42 at more.  A class has at most natoms of them.
+__host__ __device__ constexpr int stage_groups(int nb) { return (int)(stage_bytes(nb) / (27 * 16)); }
+constexpr bool stage_holds_a_class() {
+    for (int nb = 3; nb <= kMaxNb; nb += 3)
+        if (stage_groups(nb) < nb / 3) return false;
+    return true;
+}
+static_assert(stage_holds_a_class(), "k4_tables puts the groups of one class in the stage");
 
 // The +- and -- channels keep a q'' only when q''' >= q''; phase A then walks a list of
 // those q'' (16-bit indices, built per work item) instead of testing every q''.
@@ -180,14 +191,15 @@ __host__ __device__ inline Layout k4_layout_z(int kind, int NT, bool mixed, int 
     o = al16(o + (size_t)njjl * 2 + 32 * 4);  // the list, then per-warp counts of the compaction
     L.stgp = stage_passes((int)nb2);
     L.stg = (int)o;  // per staged point: the records (v, omega) of its nb branches, then those of its partner
-    o = al16(o + (size_t)stage_slots((int)nb2) * 2 * nb * 32);
+    o = al16(o + stage_bytes(nb));
     L.red = L.stg;  // the sums of the work counters, after the last work item
-    L.bgrp = stage_slots((int)nb2) * 2 * nb * 32 / (27 * 16);  // cluster groups that fit there in phase B
+    L.bgrp = stage_groups(nb);
     L.stgi = (int)o;  // per staged point: (its index, its grid coordinates packed, the partner's index)
     o = al16(o + (size_t)stage_slots((int)nb2) * 16);
     L.misc = (int)o;
     o = al16(o + 8 * 4);
-    L.total = (int)o;
+    // (a size past 2 GB must not wrap into one that fits)
+    L.total = (int)(o < (size_t)INT32_MAX ? o : (size_t)INT32_MAX);
     return L;
 }
 
@@ -272,8 +284,8 @@ __device__ __forceinline__ const float2* eig_table<true>(const DevSys& S) {
 // One step per (i,j) took 340 FP64 instructions and 140 loads per entry of the 58
 // quartic clusters of diamond, as much as the contraction itself on small grids; this
 // takes 24 FP64 instructions and 12 shared loads, plus the first step's share.  B is
-// kept in phase A's staging area, bgrp groups at a time (a class has at most natoms
-// groups, and bgrp is at least 17).  Ends with a barrier.
+// kept in phase A's staging area, bgrp groups at a time (stage_groups: at least the natoms
+// groups that a class can have).  Ends with a barrier.
 template <typename BinJ, typename Store>
 __device__ __forceinline__ void k4_tables(const DevSys& S, const DevIfc& F, const double2* kap, double2* B, int bgrp,
                                           int ch, int q0, int ii, int i, int s0, int s1, BinJ bin_j, Store store) {
