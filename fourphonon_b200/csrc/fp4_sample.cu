@@ -12,7 +12,7 @@
 // One CTA takes a chunk of samples of one (mode, channel): its threads draw
 // and filter, survivors go to a shared-memory list, and the listed processes'
 // V(4) are contracted directly over the clusters (phases from the integer lattice
-// coordinates, as in the rate kernel), in FP64 by eight lanes per process.  Per-chunk
+// coordinates, as in the rate kernel), by eight lanes per process.  Per-chunk
 // sums go to a buffer reduced afterwards in a fixed order with compensated sums.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -127,14 +127,15 @@ __device__ double2 vp4_terms(const DevSys& S, const DevIfc& F, const double2* A,
     return V;
 }
 
-// The same sum in FP32 (mixed precision): FP32 eigenvectors and root tables,
-// the cluster constants rounded to FP32 as they are read, FP32 accumulation.
-__device__ float2 vp4_direct_f(const DevSys& S, const DevIfc& F, int ch, const float2* ei, const float2* ej,
+// The same terms in FP32 (mixed precision): FP32 eigenvectors and root tables,
+// the cluster constants rounded to FP32 as they are read, each cluster's term in FP32;
+// the sum over the clusters, whose terms cancel, in FP64.
+__device__ double2 vp4_terms_f(const DevSys& S, const DevIfc& F, int ch, const float2* ei, const float2* ej,
                                const float2* ek, const float2* el, int m0, int m1, int m2, int a0, int a1, int a2,
-                               int t0, int t1, int t2) {
+                               int t0, int t1, int t2, int c0, int dc) {
     const int sj = (ch == 2) ? -1 : 1, sk = (ch == 0) ? 1 : -1;
-    float2 V = make_float2(0.f, 0.f);
-    for (int c = 0; c < F.ntri; c++) {
+    double2 V = make_double2(0.0, 0.0);
+    for (int c = c0; c < F.ntri; c += dc) {
         const int4 at = F.atoms[c];
         const int4 mj = F.mj[c], mk = F.mk[c], ml = F.ml[c];
         const float2 ph =
@@ -176,7 +177,7 @@ __device__ float2 vp4_direct_f(const DevSys& S, const DevIfc& F, int ch, const f
             A = cmacf(A, wu, I[u]);
         }
         const float mu = (float)F.mu[c];
-        V = cmacf(V, make_float2(mu * ph.x, mu * ph.y), A);
+        V = cmac(V, make_double2(mu * ph.x, mu * ph.y), make_double2(A.x, A.y));
     }
     return V;
 }
@@ -189,11 +190,12 @@ struct SEntry {
 // Draws of one item, then V(4) and the weights of the draws that survived.  About one
 // draw in a hundred does, so that an item of 1024 draws kept ten threads of 256 walking
 // the clusters while the others waited (10 % issue activity, 15 of 18 stall cycles at a
-// barrier).  An item holds up to kSChunkMax draws instead, and in FP64 eight lanes share
-// a process's clusters; lane x of the eight then weighs temperature x.  FP32 (mixed
-// precision) keeps one lane per process, whose sum runs over the clusters in order.
-// 1.3e8 draws of the 12^3 zincblende grid at four temperatures: 52.2 ms before, 5.4 ms
-// after (4.9 ms of it here).
+// barrier).  An item holds up to kSChunkMax draws instead, and eight lanes share a
+// process's clusters; lane x of the eight then weighs temperature x.  Kernel times, with
+// 1,024 draws and one thread per process, and so: 1.3e8 draws of the 12^3 zincblende grid
+// at four temperatures, FP64 48.3, 4.65 ms, mixed 33.1, 7.0; 1.4e5 draws of diamond 4^3,
+// mixed, 0.134, 0.074.  (Mixed precision with 16,384 draws and one lane per process: 8.2
+// and 0.189.)
 template <int NT, bool MIXED>
 __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
     extern __shared__ __align__(16) unsigned char smem_s[];
@@ -228,9 +230,7 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
         const double2* ei = S.eig + (size_t)(q0 * nb + i) * nb;
         unsigned long long my_n = 0;
         Comp accP = {0.0, 0.0};
-        double acc[2 * NT];  // FP32: every temperature; FP64: [0] and [NT] of temperature l8
-#pragma unroll
-        for (int x = 0; x < 2 * NT; x++) acc[x] = 0.0;
+        double acc_r = 0.0, acc_w = 0.0;  // of temperature l8
         if (!MIXED && need_v && p.a_tab && active) {  // A_c[t][s][r] of the item's mode
             for (int x = threadIdx.x; x < p.F.ntri * 27; x += blockDim.x) {
                 const int c = x / 27, o = x - c * 27;
@@ -310,9 +310,8 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
                 continue;
             }
             const size_t plane = (size_t)nptk * nb;
-            const int per = MIXED ? 32 : 4;  // processes of one warp at a time
-            for (int e0 = (threadIdx.x >> 5) * per; e0 < nq; e0 += (kSThreads / 32) * per) {
-                const int e = e0 + (MIXED ? lane : lane >> 3);
+            for (int e0 = (threadIdx.x >> 5) * 4; e0 < nq; e0 += (kSThreads / 32) * 4) {
+                const int e = e0 + (lane >> 3);
                 const bool own = e < nq;
                 const SEntry en = q[min(e, nq - 1)];
                 const int j = en.jkl & 0xff, k = (en.jkl >> 8) & 0xff, l = en.jkl >> 16;
@@ -323,47 +322,38 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
                     q_coords_t(S, en.ii, m0c, m1c, m2c);
                     q_coords_t(S, en.jj, a, b, cc);
                     q_coords_t(S, en.ss, t0, t1, t2);
-                    if (MIXED) {
-                        const float2* eif = S.eigf + (size_t)(q0 * nb + i) * nb;
-                        const float2 V = vp4_direct_f(S, p.F, ch, eif, S.eigf + (size_t)(en.ii * nb + j) * nb,
-                                                      S.eigf + (size_t)(en.jj * nb + k) * nb,
-                                                      S.eigf + (size_t)(en.ss * nb + l) * nb, m0c, m1c, m2c, a, b,
-                                                      cc, t0, t1, t2);
-                        v2 = (double)V.x * (double)V.x + (double)V.y * (double)V.y;
-                    } else {
-                        double2 V = vp4_terms(S, p.F, p.a_tab ? A : nullptr, ch, ei,
-                                              S.eig + (size_t)(en.ii * nb + j) * nb,
-                                              S.eig + (size_t)(en.jj * nb + k) * nb,
-                                              S.eig + (size_t)(en.ss * nb + l) * nb, m0c, m1c, m2c, a, b, cc, t0, t1,
-                                              t2, l8, 8);
-                        __syncwarp();
+                    const size_t r0 = (size_t)(q0 * nb + i) * nb, r1 = (size_t)(en.ii * nb + j) * nb,
+                                 r2 = (size_t)(en.jj * nb + k) * nb, r3 = (size_t)(en.ss * nb + l) * nb;
+                    double2 V;
+                    if constexpr (MIXED)
+                        V = vp4_terms_f(S, p.F, ch, S.eigf + r0, S.eigf + r1, S.eigf + r2, S.eigf + r3, m0c, m1c, m2c, a,
+                                        b, cc, t0, t1, t2, l8, 8);
+                    else
+                        V = vp4_terms(S, p.F, p.a_tab ? A : nullptr, ch, S.eig + r0, S.eig + r1, S.eig + r2, S.eig + r3,
+                                      m0c, m1c, m2c, a, b, cc, t0, t1, t2, l8, 8);
+                    __syncwarp();
 #pragma unroll
-                        for (int o = 4; o > 0; o >>= 1) {
-                            V.x += __shfl_xor_sync(0xffffffffu, V.x, o);
-                            V.y += __shfl_xor_sync(0xffffffffu, V.y, o);
-                        }
-                        v2 = V.x * V.x + V.y * V.y;
+                    for (int o = 4; o > 0; o >>= 1) {
+                        V.x += __shfl_xor_sync(0xffffffffu, V.x, o);
+                        V.y += __shfl_xor_sync(0xffffffffu, V.y, o);
                     }
+                    v2 = V.x * V.x + V.y * V.y;
                 }
                 const double g = exp(-(en.delta * en.delta) / (en.sigma * en.sigma));
                 const bool low = (w1 <= 1.25 || w2 <= 1.25 || w3 <= 1.25);
-#pragma unroll
-                for (int x = 0; x < (MIXED ? NT : 1); x++) {
-                    const int t = MIXED ? x : l8;
-                    if (own && t < p.nT) {
-                        const double* bz = p.bose + t * plane;
-                        const double f1 = bz[en.ii * nb + j], f2 = bz[en.jj * nb + k], f3 = bz[en.ss * nb + l];
-                        double bc;
-                        if (ch == 0)
-                            bc = f1 * f2 * (1 + f3) - (1 + f1) * (1 + f2) * f3;
-                        else if (ch == 1)
-                            bc = f1 * (1 + f2) * (1 + f3) - (1 + f1) * f2 * f3;
-                        else
-                            bc = (1 + f1) * (1 + f2) * (1 + f3) - f1 * f2 * f3;
-                        const double wp4 = low ? 0.0 : bc * g / en.sigma / sqrtpi / (omega * w1 * w2 * w3);
-                        acc[x] = fma(wp4, v2, acc[x]);
-                        acc[NT + x] += wp4;
-                    }
+                if (own && l8 < p.nT) {  // temperature l8
+                    const double* bz = p.bose + l8 * plane;
+                    const double f1 = bz[en.ii * nb + j], f2 = bz[en.jj * nb + k], f3 = bz[en.ss * nb + l];
+                    double bc;
+                    if (ch == 0)
+                        bc = f1 * f2 * (1 + f3) - (1 + f1) * (1 + f2) * f3;
+                    else if (ch == 1)
+                        bc = f1 * (1 + f2) * (1 + f3) - (1 + f1) * f2 * f3;
+                    else
+                        bc = (1 + f1) * (1 + f2) * (1 + f3) - f1 * f2 * f3;
+                    const double wp4 = low ? 0.0 : bc * g / en.sigma / sqrtpi / (omega * w1 * w2 * w3);
+                    acc_r = fma(wp4, v2, acc_r);
+                    acc_w += wp4;
                 }
             }
             __syncthreads();  // the list is read
@@ -373,9 +363,8 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
         double v[2 * NT + 2];
 #pragma unroll
         for (int x = 0; x < NT; x++) {
-            const bool mine = MIXED || p.mode != 2 || l8 == x;
-            v[x] = mine ? acc[(MIXED ? x : 0)] : 0.0;
-            v[NT + x] = mine ? acc[NT + (MIXED ? x : 0)] : 0.0;
+            v[x] = l8 == x ? acc_r : 0.0;
+            v[NT + x] = l8 == x ? acc_w : 0.0;
         }
         if (p.mode != 2) v[0] = accP.val();
         v[2 * NT] = (double)my_n;
