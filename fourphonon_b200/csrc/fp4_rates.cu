@@ -100,10 +100,10 @@ __global__ void __launch_bounds__(kThreads3) k3_mode(P3Params p) {
 
     // A pass takes kC3 rows of blockDim.x consecutive candidates, one of each row to a
     // thread: one barrier per 1,024 candidates (three per 256 before), and the loads stay
-    // coalesced (16^3 diamond: NP_driver's kernel 2.9 -> 2.15 ms, Ind_driver's 8.1 ->
-    // 7.15 ms).  (j, ii, k) of the thread's candidate advance by blockDim.x, without divisions.
+    // coalesced (16^3 diamond: NP_driver's kernel 2.9 -> 2.15 ms, Ind_driver's 7.7 ->
+    // 6.5 ms).  (j, ii, k) of the thread's candidate advance by blockDim.x, without divisions.
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pass = kC3 * kThreads3, dk = kThreads3 % nb, dq = kThreads3 / nb;
+    const int pass = kC3 * kThreads3, dk = kThreads3 % nb, dq = kThreads3 / nb % nptk, dj = kThreads3 / nb / nptk;
     int j = (int)threadIdx.x / per_j, ii = ((int)threadIdx.x - j * per_j) / nb,
         k = (int)threadIdx.x - j * per_j - ii * nb, buf = 0;
     for (long long base = 0; base < total; base += pass, buf ^= 32) {
@@ -132,11 +132,12 @@ __global__ void __launch_bounds__(kThreads3) k3_mode(P3Params p) {
             keep[y] = __ballot_sync(0xffffffffu, ok);
             k += dk;
             ii += dq;
+            j += dj;
             if (k >= nb) {
                 k -= nb;
                 ii++;
             }
-            while (ii >= nptk) {
+            if (ii >= nptk) {
                 ii -= nptk;
                 j++;
             }
@@ -183,7 +184,11 @@ __global__ void __launch_bounds__(kThreads3) k3_mode(P3Params p) {
             // every thread's queue write of this pass must be visible before any thread
             // reads the queue (the condition is uniform over the block)
             __syncthreads();
-            for (int e = threadIdx.x; e < qn; e += blockDim.x) {
+            // whole rounds of the block, but for the last; the rest goes to the queue's front.
+            // (A pass needs kQ3 / 2 free entries, so that a drain comes after 1,025 to 2,048;
+            // with all of them drained each time, layered 3^3 took 0.161 ms, 0.141 so.)
+            const int nd = last ? qn : qn - qn % kThreads3;
+            for (int e = threadIdx.x; e < nd; e += blockDim.x) {
                 const int xx = queue[e];
                 const int jj = xx / per_j, rem = xx - jj * per_j, q1 = rem / nb, kk = rem - q1 * nb;
                 int a, b, c;
@@ -250,7 +255,11 @@ __global__ void __launch_bounds__(kThreads3) k3_mode(P3Params p) {
                 }
             }
             __syncthreads();
-            qn = 0;
+            qn -= nd;
+            if ((int)threadIdx.x < qn) {  // (nd > kQ3 / 2 here, so the two ranges are apart)
+                queue[threadIdx.x] = queue[nd + threadIdx.x];
+                qpos[threadIdx.x] = qpos[nd + threadIdx.x];
+            }
         }
     }
     if (MODE == 0) {
