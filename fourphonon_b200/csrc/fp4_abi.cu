@@ -197,6 +197,7 @@ extern "C" int fp4_set_upload_cache(fp4_ctx* c, int enable) {
 // plain copies, then lanes that are open; fresh: a first call less 12 ms for the pinning):
 //               fresh        mapped       to the device
 //     8.5 MB    6.5,  -       2.7,  2.8    1.0, 0.9
+//      15 MB     -,   -       4.0,  3.9    0.98, 0.77
 //      31 MB   14.8,  8       7.7,  6.9    3.0, 2.3
 //     110 MB   41,   19      21.4, 19.3   14.4, 7.6
 // so below kCopyMin the threads save nothing.  Pinning the slots takes 9 to 17 ms, which
@@ -207,7 +208,7 @@ extern "C" int fp4_set_upload_cache(fp4_ctx* c, int enable) {
 // Slots of 512 KB would take half as long to pin, and a 110 MB sweep 1.1 ms longer.
 static constexpr int kCopyThreads = 8;
 static constexpr size_t kCopyChunk = (size_t)1 << 20;
-static constexpr size_t kCopyMin = (size_t)16 << 20;
+static constexpr size_t kCopyMin = (size_t)8 << 20;
 static constexpr size_t kCopyOpen = (size_t)256 << 20;
 
 void fp4_close_lanes(fp4_ctx* c) {
