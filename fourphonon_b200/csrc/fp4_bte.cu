@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(1024) k_sweep(BteParams p) {
 // memory.  k_sweep put every term of a step into the chain: 13.5 us a step on the 12^3
 // diamond grid (140 ms a sweep).  Here a step of the chain is two barriers and a few
 // hundred terms; the sweep, its symmetrisation and kappa take 17.6 ms with their copies.
-constexpr int kBlockPoints = 64;   // points of a block (one star may have more)
+constexpr int kBlockPoints = 64;   // most points of a block (one star may have more)
 constexpr int kStepThreads = 128;  // threads of k_block_steps
 
 struct StepInfo {
@@ -660,18 +660,37 @@ struct Lists4 {
 
 static size_t block_smem(int nb, int pts) { return (size_t)pts * (nb * 3 + 9) * sizeof(double); }
 
-// Cuts the irreducible points into blocks of at most kBlockPoints points (or one star),
-// and lays out their steps and, for the worst case that every term falls inside the
-// block, their listed terms; terms, steps and pts are the largest block's.  False when a
-// block's terms or points would take too much memory, or when there are more branches than
-// k_block_steps has threads: the sweep then runs on k_sweep.  (The worst case is far from
-// the listed share of about B / nptk: the 12^3 diamond grid gets 20 MB and lists 4 % of it.
-// One star of 48 points passes the limit when its modes have 350,000 processes in all.)
-static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* n_plus, const int32_t* n_minus,
-                        std::vector<int>& cut, std::vector<int>& step0, std::vector<long long>& term0, size_t& terms,
-                        size_t& steps, int& pts) {
+// Cuts the irreducible points into blocks of at most B points (or one star), and lays out
+// their steps and, for the worst case that every term falls inside the block, their listed
+// terms; terms, steps and pts are the largest block's.
+//   B: of a mode's m terms a block of B points lists m B / nptk for the chain, whose threads
+// read two of them ahead each; more are waited for.  So B is the most points whose steps
+// keep to 2 kStepThreads terms, and kBlockPoints where that is more: a block costs two
+// launches and the serial rows of k_block_sums, about 10 us and 9 ns for each of m / 2
+// processes.  3-atom cell on 8^3, B = 13 (2, 8, 16, 64 points: 17.4, 8.3, 8.8, 19.4 ms; k_sweep
+// 40.2); 8-atom cell on 4^3, B = 1, two points to a star (2, 8, 64 points: 3.3, 7.0, 76 ms;
+// k_sweep 14.2); diamond 16^3, B = 63 (32, 64 points: 38.2, 34.4 ms; k_sweep 583).
+//   False, and the sweep runs on k_sweep, where that is the cheaper one (a few points with
+// many processes, half of whose terms lie inside a star), when a block's terms or points
+// would take too much memory, or when there are more branches than k_block_steps has
+// threads.  (The worst case is far from the listed share of about B / nptk: the 12^3 diamond
+// grid gets 16 MB and lists 3 % of it.  One star of 48 points passes the limit when its
+// modes have 350,000 processes in all.)
+static bool plan_blocks(int nb, int nptk, int nlist, const int32_t* nequi, const int32_t* n_plus,
+                        const int32_t* n_minus, long long nproc, std::vector<int>& cut, std::vector<int>& step0,
+                        std::vector<long long>& term0, size_t& terms, size_t& steps, int& pts) {
     const size_t kMaxTerms = (size_t)32 << 20;  // 384 MB of indices and amplitudes
     const size_t kMaxSmem = 200 * 1024;
+    const double m = 2.0 * nproc / ((double)nb * nlist);      // a mode's terms
+    const double kBlockNs = 10000.0 + 4.5 * m;
+    const double kStepNs = 650.0, kTermNs = 3.0;              // a step of the chain, and each of its listed terms
+    const double kSweepStepNs = 1900.0, kSweepTermNs = 0.65;  // a step of k_sweep, and each of its terms
+    const int B = (int)std::max(1.0, std::min((double)kBlockPoints, 2.0 * kStepThreads * nptk / (m + 1.0)));
+    double blocks_ns = 0.0, sweep_ns = 0.0;
+    auto add_cost = [&](double points, double all) {  // of a block whose steps have `all` terms together
+        blocks_ns += kBlockNs + points * nb * kStepNs + kTermNs * all * points / nptk;
+        sweep_ns += points * nb * kSweepStepNs + kSweepTermNs * all;
+    };
     cut.assign(1, 0);
     step0.assign(nlist + 1, 0);
     term0.assign((size_t)nb * nlist, 0);
@@ -682,7 +701,8 @@ static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* 
     for (int ll = 0; ll < nlist; ll++) {
         size_t lt = 0;
         for (int i = 0; i < nb; i++) lt += (size_t)2 * ((size_t)n_plus[ll * nb + i] + n_minus[ll * nb + i]) * nequi[ll];
-        if (ll > cut.back() && (bp + nequi[ll] > kBlockPoints || bt + lt > kMaxTerms)) {
+        if (ll > cut.back() && (bp + nequi[ll] > B || bt + lt > kMaxTerms)) {
+            add_cost(bp, (double)bt);
             cut.push_back(ll);
             bt = 0;
             bp = 0;
@@ -697,8 +717,9 @@ static bool plan_blocks(int nb, int nlist, const int32_t* nequi, const int32_t* 
         steps = std::max(steps, (size_t)(step0[ll + 1] - step0[cut.back()]));
         pts = std::max(pts, bp);
     }
+    add_cost(bp, (double)bt);
     cut.push_back(nlist);
-    return nb <= kStepThreads && terms <= kMaxTerms && block_smem(nb, pts) <= kMaxSmem;
+    return blocks_ns < sweep_ns && nb <= kStepThreads && terms <= kMaxTerms && block_smem(nb, pts) <= kMaxSmem;
 }
 
 static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int32_t* nequi, const int32_t* allequi,
@@ -858,7 +879,7 @@ static int run_sweep(fp4_ctx* c, const fp4_globals* g, int32_t nlist, const int3
     std::vector<long long> term0;
     size_t terms = 0, steps = 0;
     int pts = 0;
-    bool blocks = !l4 && plan_blocks(nb, nlist, nequi, n_plus, n_minus, cut, step0, term0, terms, steps, pts);
+    bool blocks = !l4 && plan_blocks(nb, nptk, nlist, nequi, n_plus, n_minus, op[nm] + om[nm], cut, step0, term0, terms, steps, pts);
     // [slot_of | step0] and [term0], [records], [coef], [idx] in one buffer
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t o1 = up((size_t)nptk * sizeof(int)), o2 = o1 + up((nlist + 1) * sizeof(int)),

@@ -47,6 +47,7 @@ def _compare(s, n_plus, n_minus, seed=1):
     try:
         F0 = ctx.iteration0(s, tau)
         got = ctx.iteration(s, F0.copy(), tau, n_plus, n_minus, lists)
+        launches = ctx.stats()[4]
     finally:
         ctx.close()
     want = O.Oracle(s).iteration(F0.copy(), tau, n_plus, n_minus, lists)
@@ -54,6 +55,7 @@ def _compare(s, n_plus, n_minus, seed=1):
     # most the largest |F|; the sweep at most doubles what a step brings in
     rtol = 2.0 * EPS * 2 * int(max(n_plus.max(), n_minus.max()) + 64)
     assert np.abs(got - want).max() <= rtol * np.abs(want).max()
+    return launches
 
 
 @pytest.mark.parametrize("natoms", [42, 43, 86])
@@ -116,3 +118,13 @@ def test_no_memory_for_the_listed_terms():
     finally:
         del hog
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("grid,natoms,count,launches", [
+    ((2, 2, 2), 2, 10, 3),       # all points in one block: its mark, its sums, its chain
+    ((4, 4, 4), 8, 2_800, 17),   # many processes per mode: each of the eight stars by itself
+    ((2, 2, 2), 2, 20_000, 1)])  # half of a star's many terms lie inside it: the sequential kernel
+def test_the_size_of_the_blocks(grid, natoms, count, launches):
+    s = _solve(grid, natoms)
+    n = np.full(s.nmodes, count, dtype=np.int32)
+    assert _compare(s, n, n.copy()) == launches
