@@ -44,7 +44,6 @@ struct PSParams {
     unsigned long long seed;
     int chunk;   // samples per item
     int nchunk;  // chunks per (mode, channel)
-    int a_tab;   // 1: the clusters contracted with the mode's eigenvector fit in shared memory
     int mode;    // 0: counts and P4, 2: rates and WP4
     int nitems;
     int* work_counter;
@@ -68,8 +67,9 @@ __device__ __forceinline__ int draw_k(unsigned long long base, int k, int range)
 // (Vp_pp/pm/mm, processes.f90:142-330):
 //   sum_c mu_c exp(2 pi i (s_j n'.m_j + s_k n''.m_k - n'''.m_l)/N)
 //         sum_{t,s,r} A_c[t][s][r] e~'_j[t] e~''_k[s] conj(e'''_l[r]),
-// A_c[t][s][r] = sum_u Psi_c[u][t][s][r] e_i[u], from the table A of the item's mode or
-// (A == nullptr) formed here.
+// A_c[t][s][r] = sum_u Psi_c[u][t][s][r] e_i[u], from the table A of the item's mode
+// (TABLE) or formed here.
+template <bool TABLE>
 __device__ double2 vp4_terms(const DevSys& S, const DevIfc& F, const double2* A, int ch, const double2* ei,
                              const double2* ej, const double2* ek, const double2* el, int m0, int m1, int m2, int a0,
                              int a1, int a2, int t0, int t1, int t2, int c0, int dc) {
@@ -90,7 +90,6 @@ __device__ double2 vp4_terms(const DevSys& S, const DevIfc& F, const double2* A,
             L[x] = cconj(el[3 * at.w + x]);
         }
         const double* psi = F.phi + (size_t)c * 81;
-        const double2* Ac = A ? A + (size_t)c * 27 : nullptr;
         double2 B = make_double2(0.0, 0.0);
 #pragma unroll 1
         for (int t = 0; t < 3; t++) {
@@ -104,8 +103,8 @@ __device__ double2 vp4_terms(const DevSys& S, const DevIfc& F, const double2* A,
                 for (int r = 0; r < 3; r++) {
                     const int o = (t * 3 + s) * 3 + r;
                     double2 f;
-                    if (A) {
-                        f = Ac[o];
+                    if (TABLE) {
+                        f = A[(size_t)c * 27 + o];
                     } else {
                         f = make_double2(0.0, 0.0);
 #pragma unroll
@@ -125,6 +124,22 @@ __device__ double2 vp4_terms(const DevSys& S, const DevIfc& F, const double2* A,
         V = cmac(V, w, B);
     }
     return V;
+}
+
+// The table of a mode with eigenvector ei: A_c[t][s][r] of every cluster, by the whole block.
+__device__ void mode_table(const DevIfc& F, const double2* ei, double2* A) {
+    for (int x = threadIdx.x; x < F.ntri * 27; x += blockDim.x) {
+        const int c = x / 27, o = x - c * 27;
+        const double* f = F.phi + (size_t)c * 81 + o;
+        const double2* e = ei + 3 * F.atoms[c].x;
+        double2 a = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            a.x = fma(f[u * 27], e[u].x, a.x);
+            a.y = fma(f[u * 27], e[u].y, a.y);
+        }
+        A[x] = a;
+    }
 }
 
 // The same terms in FP32 (mixed precision): FP32 eigenvectors and root tables,
@@ -182,6 +197,10 @@ __device__ double2 vp4_terms_f(const DevSys& S, const DevIfc& F, int ch, const f
     return V;
 }
 
+// How a kernel forms V(4): FP64 from the table of the item's mode, FP64 from the clusters
+// where there is no room for it, or in mixed precision.
+enum { kTable, kDirect, kMixed };
+
 struct SEntry {
     int ii, jj, ss, jkl;
     double sigma, delta;
@@ -196,7 +215,7 @@ struct SEntry {
 // at four temperatures, FP64 48.3, 4.65 ms, mixed 33.1, 7.0; 1.4e5 draws of diamond 4^3,
 // mixed, 0.134, 0.074.  (Mixed precision with 16,384 draws and one lane per process: 8.2
 // and 0.189.)
-template <int NT, bool MIXED>
+template <int NT, int SUM>
 __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
     extern __shared__ __align__(16) unsigned char smem_s[];
     __shared__ int s_cnt, s_item;
@@ -227,24 +246,10 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
         const bool active = (omega != 0.0) && (omega <= S.omega_max);
         const long long c0 = (long long)chunk * p.chunk;
         const long long c1 = min(c0 + (long long)p.chunk, p.nsamples);
-        const double2* ei = S.eig + (size_t)(q0 * nb + i) * nb;
         unsigned long long my_n = 0;
         Comp accP = {0.0, 0.0};
         double acc_r = 0.0, acc_w = 0.0;  // of temperature l8
-        if (!MIXED && need_v && p.a_tab && active) {  // A_c[t][s][r] of the item's mode
-            for (int x = threadIdx.x; x < p.F.ntri * 27; x += blockDim.x) {
-                const int c = x / 27, o = x - c * 27;
-                const double* f = p.F.phi + (size_t)c * 81 + o;
-                const double2* e = ei + 3 * p.F.atoms[c].x;
-                double2 a = make_double2(0.0, 0.0);
-#pragma unroll
-                for (int u = 0; u < 3; u++) {
-                    a.x = fma(f[u * 27], e[u].x, a.x);
-                    a.y = fma(f[u * 27], e[u].y, a.y);
-                }
-                A[x] = a;
-            }
-        }
+        bool tab = SUM != kTable || !need_v;  // the table of the item's mode is there, or none is wanted
         for (long long base = c0; active && base < c1;) {
             for (int rd = 0; rd < kSRounds && base < c1; rd++, base += blockDim.x) {
                 const long long it = base + threadIdx.x;
@@ -309,6 +314,11 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
                 __syncthreads();  // every thread has read the count
                 continue;
             }
+            if (!tab && nq > 0) {  // an item without survivors needs no table
+                mode_table(p.F, S.eig + (size_t)(q0 * nb + i) * nb, A);
+                tab = true;
+                __syncthreads();
+            }
             const size_t plane = (size_t)nptk * nb;
             for (int e0 = (threadIdx.x >> 5) * 4; e0 < nq; e0 += (kSThreads / 32) * 4) {
                 const int e = e0 + (lane >> 3);
@@ -325,12 +335,12 @@ __global__ void __launch_bounds__(kSThreads, 2) k4_sample(PSParams p) {
                     const size_t r0 = (size_t)(q0 * nb + i) * nb, r1 = (size_t)(en.ii * nb + j) * nb,
                                  r2 = (size_t)(en.jj * nb + k) * nb, r3 = (size_t)(en.ss * nb + l) * nb;
                     double2 V;
-                    if constexpr (MIXED)
+                    if constexpr (SUM == kMixed)
                         V = vp4_terms_f(S, p.F, ch, S.eigf + r0, S.eigf + r1, S.eigf + r2, S.eigf + r3, m0c, m1c, m2c, a,
                                         b, cc, t0, t1, t2, l8, 8);
                     else
-                        V = vp4_terms(S, p.F, p.a_tab ? A : nullptr, ch, S.eig + r0, S.eig + r1, S.eig + r2, S.eig + r3,
-                                      m0c, m1c, m2c, a, b, cc, t0, t1, t2, l8, 8);
+                        V = vp4_terms<SUM == kTable>(S, p.F, A, ch, S.eig + r0, S.eig + r1, S.eig + r2, S.eig + r3, m0c,
+                                                     m1c, m2c, a, b, cc, t0, t1, t2, l8, 8);
                     __syncwarp();
 #pragma unroll
                     for (int o = 4; o > 0; o >>= 1) {
@@ -652,11 +662,11 @@ static int run_sample(fp4_ctx* c, int mode, int nT, const double* temps, int64_t
     const bool mixed = mode == 2 && c->precision != FP4_PREC_FP64;
     size_t smem = mode == 2 ? kSList * sizeof(SEntry) : 0;
     const size_t a_bytes = (size_t)p.F.ntri * 27 * sizeof(double2);
-    p.a_tab = mode == 2 && !mixed && !S.onlyharmonic && smem + a_bytes <= 200 * 1024;
-    if (p.a_tab) smem += a_bytes;
+    const bool table = mode == 2 && !mixed && !S.onlyharmonic && smem + a_bytes <= 200 * 1024;
+    if (table) smem += a_bytes;
 #define FP4_KS(NTV)                                                                                                \
     {                                                                                                              \
-        auto kernel = mixed ? k4_sample<NTV, true> : k4_sample<NTV, false>;                                        \
+        auto kernel = mixed ? k4_sample<NTV, kMixed> : table ? k4_sample<NTV, kTable> : k4_sample<NTV, kDirect>;                                        \
         CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                  \
         kernel<<<nblocks, kSThreads, smem, c->stream>>>(p);                                                        \
     }

@@ -60,3 +60,11 @@ def test_more_clusters_than_the_table_holds(shell, nT):
     s = S.build_solve(C.layered_rhombohedral(), (2, 2, 2), (300.0,), 20240602, fc3_shell=2, fc4_shell=shell)
     assert s.ifc4.ntri > 398
     _compare(s, 20_000, 5, [300.0 + 200.0 * t for t in range(nT)])
+
+
+@pytest.mark.parametrize("cell,nsamples", [("random7", 100), ("random7", 5_000), ("diamond", 100)])
+def test_items_with_few_or_no_survivors(cell, nsamples):
+    """The table of the item's mode is built for an item's first survivor."""
+    s = H.cached_solve(cell, (2, 2, 2))
+    kept = _compare(s, nsamples, 9, [300.0])
+    assert kept < 3 * s.nmodes * nsamples
