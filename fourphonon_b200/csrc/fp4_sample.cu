@@ -658,8 +658,8 @@ static int run_sample(fp4_ctx* c, int mode, int nT, const double* temps, int64_t
     p.err = c->b_err.as<int>();
     const int nblocks = (int)std::min<int64_t>(nitems, (int64_t)c->sm_count * 8);
     CK(cudaEventRecord(c->evk0, c->stream));
-    // mixed precision: the V(4) sums in FP32 (the draws, filter, weights and sums stay FP64)
-    const bool mixed = mode == 2 && c->precision != FP4_PREC_FP64;
+    // mixed precision: the V(4) terms in FP32 (the draws, filter, weights and sums stay FP64)
+    const bool mixed = mode == 2 && c->precision != FP4_PREC_FP64 && !S.onlyharmonic;
     size_t smem = mode == 2 ? kSList * sizeof(SEntry) : 0;
     const size_t a_bytes = (size_t)p.F.ntri * 27 * sizeof(double2);
     const bool table = mode == 2 && !mixed && !S.onlyharmonic && smem + a_bytes <= 200 * 1024;
