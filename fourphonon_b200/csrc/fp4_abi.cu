@@ -186,12 +186,11 @@ extern "C" int fp4_set_upload_cache(fp4_ctx* c, int enable) {
 // A process list is tens to hundreds of MB of pageable memory, and an output list is
 // often fresh, its pages not yet mapped.  A plain copy runs through the driver's staging
 // buffer on one thread, which also takes every page fault.  Here up to kCopyThreads
-// threads take chunks in turn, each through a lane of its own (a stream and two pinned
-// slots), so that the transfers, the host copies and the page faults of different chunks
-// overlap.
-//   The lanes' streams wait for an event that the calling thread records on c->stream:
-// the caller's handle itself is used on the calling thread only, since cudaStreamPerThread
-// means another stream in each thread.
+// threads take chunks in turn, each through a lane of its own (two pinned slots), so that
+// the transfers, the host copies and the page faults of different chunks overlap.
+//   The transfers go on a stream of their own, which waits for an event that the calling
+// thread records on c->stream: the caller's handle itself is used on the calling thread
+// only, since cudaStreamPerThread means another stream in each thread.
 //   When (16 usable processors; ms of Ind_driver, whose lists go to the host, into pages
 // that are fresh or already mapped, and of a Jacobi sweep, whose lists go to the device;
 // plain copies, then lanes that are open; fresh: a first call less 12 ms for the pinning):
@@ -215,9 +214,10 @@ void fp4_close_lanes(fp4_ctx* c) {
     for (auto& l : c->lanes) {
         for (auto& v : l.done)
             if (v) cudaEventDestroy(v);
-        if (l.stream) cudaStreamDestroy(l.stream);
     }
     c->lanes.clear();
+    if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+    c->copy_stream = nullptr;
     if (c->ev_copy) cudaEventDestroy(c->ev_copy);
     c->ev_copy = nullptr;
     if (c->slots) cudaFreeHost(c->slots);
@@ -228,11 +228,11 @@ static bool open_lanes(fp4_ctx* c, int n) {
     cudaError_t e = cudaMallocHost(&c->slots, (size_t)n * 2 * kCopyChunk);
     if (e != cudaSuccess) c->slots = nullptr;
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_copy, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
     c->lanes.resize(n);
     for (int x = 0; x < n; x++) {
         CopyLane& l = c->lanes[x];
         l.slot = c->slots + (size_t)x * 2 * kCopyChunk;
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
         for (auto& v : l.done)
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
     }
@@ -283,6 +283,7 @@ int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
         return FP4_OK;
     }
     CK(cudaEventRecord(c->ev_copy, c->stream));
+    CK(cudaStreamWaitEvent(c->copy_stream, c->ev_copy, 0));
     std::vector<size_t> first(n + 1, 0);  // chunks before each copy
     for (int x = 0; x < n; x++) first[x + 1] = first[x] + (list[x].bytes + kCopyChunk - 1) / kCopyChunk;
     std::atomic<size_t> next{0};
@@ -290,7 +291,6 @@ int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
     auto work = [&](int id) {
         const CopyLane& lane = c->lanes[id];
         cudaError_t e = cudaSetDevice(c->device);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(lane.stream, c->ev_copy, 0);
         struct Pending {
             void* host;
             size_t bytes;
@@ -314,15 +314,15 @@ int fp4_copy_lists(fp4_ctx* c, const HostCopy* list, int n, bool to_host) {
             finish(s);
             if (e != cudaSuccess) break;
             if (!to_host) memcpy(slot(s), h, m);
-            e = cudaMemcpyAsync(to_host ? slot(s) : d, to_host ? d : slot(s), m, kind, lane.stream);
-            if (e == cudaSuccess) e = cudaEventRecord(lane.done[s], lane.stream);
+            e = cudaMemcpyAsync(to_host ? slot(s) : d, to_host ? d : slot(s), m, kind, c->copy_stream);
+            if (e == cudaSuccess) e = cudaEventRecord(lane.done[s], c->copy_stream);
             pend[s] = {h, m};
         }
         finish(0);
         finish(1);
         if (e != cudaSuccess) {  // nothing of this lane stays in flight behind an error
             failed = (int)e;
-            cudaStreamSynchronize(lane.stream);
+            cudaStreamSynchronize(c->copy_stream);
         }
     };
     std::vector<std::thread> pool;

@@ -52,7 +52,6 @@ struct IfcTables {
 
 // One host thread's way between pageable and device memory.
 struct CopyLane {
-    cudaStream_t stream = nullptr;
     cudaEvent_t done[2] = {nullptr, nullptr};  // the last transfer of each slot
     unsigned char* slot = nullptr;             // two pinned slots
 };
@@ -76,10 +75,11 @@ struct fp4_ctx {
     DevBuffer b_energy, b_velocity, b_wv, b_eigraw, b_eig, b_eigf, b_list, b_qc, b_root[3], b_rootf[3];
     DevBuffer b_temps, b_bose, b_wb, b_out, b_out4, b_lists, b_gamma, b_off, b_counts;
     DevBuffer b_queue, b_part, b_work, b_err, b_stats;
-    std::vector<CopyLane> lanes;       // of fp4_copy_lists, once they are worth their pinning
-    unsigned char* slots = nullptr;    // their pinned memory
-    cudaEvent_t ev_copy = nullptr;     // what c->stream held when the lanes' copies began
-    size_t list_bytes = 0;             // bytes of large lists copied so far, those to the host three times
+    std::vector<CopyLane> lanes;         // of fp4_copy_lists, once they are worth their pinning
+    unsigned char* slots = nullptr;      // their pinned memory
+    cudaStream_t copy_stream = nullptr;  // of their transfers
+    cudaEvent_t ev_copy = nullptr;       // what c->stream held when the lanes' copies began
+    size_t list_bytes = 0;               // bytes of large lists copied so far, those to the host three times
     DevBuffer b_tcplan, b_wtab;  // tensor-core contraction: its plan and phase rows
     bool last_tc = false;        // the last four-phonon RTA call ran its contraction on the tensor cores
     DevBuffer b_bte[13];  // [12]: the new iterate of a Jacobi sweep
