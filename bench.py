@@ -797,7 +797,7 @@ def run_bte(ctx, s, rate4, T, maxiter=200):
             "jacobi": {"iterations": itj, "sweep_kernel_ms_mean": float(np.mean(jac_ms)),
                        "sweep_wall_s_mean": (t4 - t3) / itj, "loop_wall_s": t4 - t3, "kappa_converged": k_j,
                        "kappa_rel_diff_vs_gauss_seidel": abs(k_j - k_gs) / abs(k_gs)},
-            "note": "Gauss-Seidel: one CTA runs each sweep in the reference's order; Jacobi: every step of a "
+            "note": "Gauss-Seidel: a chain of steps in the reference's order; Jacobi: every step of a "
                     "sweep at once (fp4_iteration_jacobi); wall times include the host calls that pass the lists"}
 
 

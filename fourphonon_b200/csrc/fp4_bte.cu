@@ -202,9 +202,9 @@ __global__ void __launch_bounds__(1024) k_sweep(BteParams p) {
 // which k_block_sums forms for every step of the block at once on the whole GPU, and
 // the few at the block's points (about 2 n B / nptk of a mode's 2 n terms for B points),
 // which it lists and k_block_steps adds in the reference's step order from shared
-// memory.  k_sweep put every term of a step into the chain: 13.5 us a step on the 12^3
-// diamond grid (140 ms a sweep).  Here a step of the chain is two barriers and a few
-// hundred terms; the sweep, its symmetrisation and kappa take 17.6 ms with their copies.
+// memory.  k_sweep puts every term of a step into the chain: 12.5 us a step on the 12^3
+// diamond grid (130 ms a sweep).  Here a step of the chain is two barriers and a few
+// hundred terms, and the sweep's kernels take 13.0 ms.
 constexpr int kBlockPoints = 64;   // most points of a block (one star may have more)
 constexpr int kStepThreads = 128;  // threads of k_block_steps
 

@@ -5,9 +5,10 @@
 //   * the valid sums s_ij = w_i +- w'_j are rank-sorted in shared memory;
 //   * phase A walks every (q'', k, l) once: q''' from integer grid
 //     arithmetic, the channel's restrictions, sigma(v''-v''') in base_sigma's
-//     exact operation order (computed once for all (i,j)), a binary search for
-//     the window of s_ij that can pass the 1-sigma test, and the exact test in
-//     the reference's operation order.  Survivors are queued per (i,j);
+//     exact operation order (computed once for all (i,j)), the window of s_ij
+//     that can pass the 1-sigma test from a table of cells over their range, and
+//     the exact test in the reference's operation order.  Survivors are queued
+//     per (i,j);
 //   * phase B (a function of its own, with its own registers) builds, per branch i, the
 //     reciprocal cluster table
 //         Z_p^{(ij)}[s][r] = sum_{c in p} kappa_c sum_{u,t} Psi_c[u][t][s][r] e_i[u] e~'_j[t]
@@ -21,8 +22,8 @@
 // Per-(work item, branch, temperature) partial sums are reduced afterwards in
 // a fixed order with compensated summation (k4_reduce).
 //
-// What bounds it (12^3 diamond, FP64, two temperatures; 1.09 s before phase B's tables,
-// loads and sums were rearranged, 0.93 s now): no single unit.  Builds that leave one
+// What bounds it (12^3 diamond, FP64, two temperatures: 0.89 s; 1.09 s with phase B's tables
+// in one step and each eigenvector row read twice): no single unit.  Builds that leave one
 // part out put the class loop at 40 % of phase B, the gathers of the two eigenvector
 // rows at 16 %, the weights at 16 %, the tables at 5 %.  On 8^3 the load pipe is 61 %
 // busy, FP64 28 %, issue 45 %; the top stalls are fixed latency and loads.  More warps
@@ -106,8 +107,11 @@ struct K4Shared {
 // queue headroom within the capacity the host reserves.
 constexpr int kStageSlots = 32;
 
-// Cells of the lookup table over the range of the sorted pair sums (phase A): with 36
-// sums of 2-atom cells a window then holds 0.1 to 0.2 sums that the exact test drops.
+// Cells of the lookup table over the range of the sorted pair sums (phase A).  A window is
+// rounded outwards to whole cells, so that it holds the sums of at most two cells that the
+// exact test drops: of the nb^2 sums 0.1 to 0.2 with two atoms (36 sums), about one with
+// five (225), 3.5 with ten (900), beside windows that grow with the sums.  Any number is
+// right; 256 cells take 516 bytes and one round of the block to fill.
 constexpr int kCells = 256;
 __host__ __device__ constexpr int stage_passes(int nb2) {
     int P = 8;
@@ -164,7 +168,11 @@ __host__ __device__ inline Layout k4_layout_z(int kind, int NT, bool mixed, int 
     // counting: one copy of the per-branch count and phase-space sum per thread while
     // three CTAs per SM fit (a sum into a thread's own word needs no atomic; an FP64 atomic
     // on shared memory is a loop of compare-and-swaps), else one per warp (counting, 10^3
-    // diamond: 63.2 ms with a copy per warp and two divisions per process, 48.6 ms so)
+    // diamond: 63.2 ms with a copy per warp and two divisions per process, 48.6 ms so).
+    // They come before the list of q'', which k4_layout drops where both do not fit (9
+    // branches from 24^3, 12 from 22^3, 15 from 17^3 on): per thread without the list, per
+    // warp with it, random 5-atom 17^3 1.28, 1.38 s, layered 22^3 3.97, 4.51 s, random 4-atom
+    // 22^3 2.92, 2.90 s, random 3-atom 24^3 2.51, 2.42 s (six irreducible points each).
     L.priv = kind == 0 && (size_t)nb * kThreads * 12 <= 48 * 1024;
     const size_t ncopy = (kind == 0) ? (L.priv ? kThreads : kThreads / 32) : 1;
     L.pacc = (int)o;

@@ -215,9 +215,9 @@ int fp4_iteration(fp4_ctx *ctx, const fp4_globals *g, int32_t nlist, const int32
  * update is Gauss-Seidel, Src/iterations.f90:34-92): same arguments and
  * layouts; every step of the sweep reads the F_n passed in and the new F_n
  * (with the site symmetrizers applied) is returned in f_n.  All steps run in
- * parallel on the device, so a sweep costs milliseconds where the in-order
- * sweep keeps one CTA busy; the iteration converges to the same kappa in more
- * sweeps.  Three-phonon processes only.
+ * parallel on the device, while the in-order sweep has a serial chain of steps
+ * (about ten times as long on a 16^3 grid); the iteration converges to the same
+ * kappa in more sweeps.  Three-phonon processes only.
  */
 int fp4_iteration_jacobi(fp4_ctx *ctx, const fp4_globals *g, int32_t nlist, const int32_t *nequi,
                          const int32_t *allequi, const int32_t *typeofsym, int32_t nsymm_rot, const int32_t *id_equi,
